@@ -19,7 +19,7 @@
 //      |adjust_direction(r_i, r_j)|^2 < (cutoff (1 + margin))^2.
 // The lists hold both directions of every pair (full lists); a pair (a, b) is
 // present iff the reference's half list holds (min(a,b), max(a,b)).
-#include "kernels.cuh"
+#include "list_build.cuh"
 
 namespace mjg {
 
@@ -222,234 +222,26 @@ __global__ void __launch_bounds__(TPB) k_slots_setup(Arena a, TermArrays t)
         const double4 r = a.pos[i];
         t.slot_particle[s] = i;
         t.slot_of[i]       = s;
-        t.slot_lead[s]     = t.part_lead[p];
         t.slot_sys[s]      = w.x;
         t.slot_pd[s]       = make_double4(r.x, r.y, r.z, t.part_p0[p]);
         if(t.part_p1) {t.slot_p1[s] = t.part_p1[p];}
     }
 }
 
-// A slot's exclusion row staged in shared memory once per slot: the CSR row of
-// particle i holds every particle excluded together with i (the relation is
-// symmetric: topology distance and molecule rules; i itself included), so
-// is_excluded(min(i, j), max(i, j)) is "j is in i's row" -- a comparison
-// against the staged row instead of a chain of dependent loads per candidate.
-// Rows longer than EXMAX are scanned in global memory as before.
-constexpr int EXMAX = 16;
-struct ExRow {
-    int n;              // entries staged, or -1: the row is longer than EXMAX
-    int mol;            // molecule of particle i
-    int v[EXMAX];       // sorted excluded partners of i
-};
-// lanes [0, nl) of the slot's group stage particle i's row (every lane of the
-// group must call it, then synchronise the group before reading the row)
-__device__ __forceinline__ void stage_ex_row(const Arena& a, int g, int i, int gl, int nl, ExRow& r)
-{
-    const long long b = a.ex_start[g][i], e = a.ex_start[g][i + 1];
-    const int n = (int)(e - b);
-    if(gl == 0) {r.n = n <= EXMAX ? n : -1; r.mol = a.mol[i];}
-    if(n <= EXMAX) {for(int k = gl; k < n; k += nl) {r.v[k] = a.ex_idx[g][b + k];}}
-}
-__device__ __forceinline__ bool is_excluded(const Arena& a, int g, int ignore_mol, int i, int j);
-// is_excluded(min(i, j), max(i, j)) for the slot's particle i and candidate j
-__device__ __forceinline__ bool excluded_staged(const Arena& a, int g, int ignore_mol, const ExRow& r, int i, int j)
-{
-    if(ignore_mol != IGN_NOTHING)
-    {
-        const int mj = a.mol[j];
-        if(ignore_mol == IGN_SELF   && r.mol == mj) {return true;}
-        if(ignore_mol == IGN_OTHERS && r.mol != mj) {return true;}
-    }
-    if(r.n < 0) {return is_excluded(a, g, IGN_NOTHING, i < j ? i : j, i < j ? j : i);}
-    for(int k = 0; k < r.n; ++k)
-    {
-        const int x = r.v[k];
-        if(x > j) {break;}
-        if(x == j) {return true;}
-    }
-    return false;
-}
-
-__device__ __forceinline__ bool is_excluded(const Arena& a, int g, int ignore_mol, int i, int j)
-{
-    if(ignore_mol == IGN_SELF   && a.mol[i] == a.mol[j]) {return true;}
-    if(ignore_mol == IGN_OTHERS && a.mol[i] != a.mol[j]) {return true;}
-    const long long b = a.ex_start[g][i], e = a.ex_start[g][i + 1];
-    for(long long q = b; q < e; ++q)
-    {
-        const int x = a.ex_idx[g][q];
-        if(x > j) {break;}
-        if(x == j) {return true;}
-    }
-    return false;
-}
-
-// Half lists keep a pair in the list of its lower slot only: a stencil cell's
-// slot range [start, start + count) is cut to the slots above s (slots are in
-// cell order, so a cell is one range), which leaves the full list's words
-// above s in their order.  The full lists are symmetric (the distance test,
-// the leading-participant rule and the exclusions do not depend on which
-// partner asks), so every pair of them is in exactly one half list.
-__device__ __forceinline__ void clip_half(int& start, int& count, int s)
-{
-    const int lo = max(start, s + 1);
-    count = max(0, start + count - lo);
-    start = lo;
-}
-
-// One warp per slot.  The 27 stencil cells (in the reference's order: z, y, x
-// from -1 to +1) are flattened into one candidate sequence that the 32 lanes
-// walk together; the distance test reads the cell-ordered slot coordinates
-// (consecutive candidates are consecutive in memory), the topology checks run
-// only for candidates inside the list radius, and an ordered ballot
-// compaction keeps the output order identical to a serial walk.
-__global__ void __launch_bounds__(TPB) k_build_list(Arena a, int g, TermArrays t)
-{
-    const int n = t.work[0];
-    const int cap = t.cap;
-    const long long np = t.np;
-    const int lane = threadIdx.x & 31;
-    const unsigned full = 0xffffffffu;
-    // every warp of the grid takes the next (chunk, slot) pair, so that all
-    // warps have work even when only a few systems rebuild
-    __shared__ ExRow ex_rows[TPB / 32];
-    ExRow& exr = ex_rows[threadIdx.x >> 5];
-    const long long nwork = (long long)n * CHUNK;
-    const long long wstride = (long long)gridDim.x * (TPB / 32);
-    for(long long gw = (long long)blockIdx.x * (TPB / 32) + (threadIdx.x >> 5); gw < nwork; gw += wstride)
-    {
-        const int4 w = t.part_chunks[gw / CHUNK];
-        const int s = w.y + (int)(gw % CHUNK);
-        if(s >= w.z) {continue;}
-        const int sys = w.x;
-        const SysDev& S = a.sys[sys];
-        const GlobalParams& G = S.g[g];
-        const bool periodic = S.boundary == B_PERIODIC;
-        const int dx_ = G.dims[0], dy_ = G.dims[1], dz_ = G.dims[2];
-        const bool wrap = periodic || G.hashed;
-        const double rl2 = G.rl2;
-        {
-            const int i = t.slot_particle[s];
-            const bool lead_i = t.slot_lead[s] != 0;
-            const double4 ri = t.slot_pd[s];
-            __syncwarp();                        // the previous slot's row is no longer read
-            stage_ex_row(a, g, i, lane, 32, exr);
-            __syncwarp();
-            const int cx = cell_coord(ri.x, G, 0);
-            const int cy = cell_coord(ri.y, G, 1);
-            const int cz = cell_coord(ri.z, G, 2);
-            // this lane's stencil cell
-            int cstart = 0, ccount = 0;
-            if(lane < 27)
-            {
-                int x = cx + lane % 3 - 1, y = cy + (lane / 3) % 3 - 1, z = cz + lane / 9 - 1;
-                bool inside = true;
-                if(wrap)
-                {
-                    x = x < 0 ? x + dx_ : (x >= dx_ ? x - dx_ : x);
-                    y = y < 0 ? y + dy_ : (y >= dy_ ? y - dy_ : y);
-                    z = z < 0 ? z + dz_ : (z >= dz_ ? z - dz_ : z);
-                }
-                else if(x < 0 || y < 0 || z < 0 || x >= dx_ || y >= dy_ || z >= dz_) {inside = false;}
-                if(inside)
-                {
-                    const int cell = G.cell_off + x + dx_ * (y + dy_ * z);
-                    cstart = t.cell_start[cell];
-                    ccount = t.cell_count[cell];
-                    if(t.half) {clip_half(cstart, ccount, s);}
-                }
-            }
-            int incl = ccount;
-#pragma unroll
-            for(int o = 1; o < 32; o <<= 1)
-            {
-                const int y = __shfl_up_sync(full, incl, o);
-                if(lane >= o) {incl += y;}
-            }
-            const int excl = incl - ccount;
-            const int total = __shfl_sync(full, incl, 31);
-            int count = 0;
-            for(int base = 0; base < total; base += 32)
-            {
-                const int k = base + lane;
-                // cell of candidate k: the last stencil lane whose range starts at or before k
-                int L = 0;
-#pragma unroll
-                for(int b = 16; b > 0; b >>= 1)
-                {
-                    const int cand = L + b;
-                    const int e = __shfl_sync(full, excl, cand < 32 ? cand : 31);
-                    if(cand < 27 && e <= k) {L = cand;}
-                }
-                const int q = __shfl_sync(full, cstart, L) + (k - __shfl_sync(full, excl, L));
-                bool keep = false;
-                if(k < total && q != s)
-                {
-                    const double4 rj = t.slot_pd[q];
-                    double ddx = __dsub_rn(rj.x, ri.x);
-                    double ddy = __dsub_rn(rj.y, ri.y);
-                    double ddz = __dsub_rn(rj.z, ri.z);
-                    if(periodic)
-                    {
-                        ddx = min_image(ddx, S.halfw[0], S.width[0]);
-                        ddy = min_image(ddy, S.halfw[1], S.width[1]);
-                        ddz = min_image(ddz, S.halfw[2], S.width[2]);
-                    }
-                    const double l2 = __dadd_rn(__dadd_rn(__dmul_rn(ddx, ddx), __dmul_rn(ddy, ddy)), __dmul_rn(ddz, ddz));
-                    if(l2 < rl2)
-                    {
-                        const int j = t.slot_particle[q];
-                        const bool lead_lo = (i < j) ? lead_i : (t.slot_lead[q] != 0);
-                        keep = lead_lo && !excluded_staged(a, g, G.ignore_mol, exr, i, j);
-                    }
-                }
-                const unsigned m = __ballot_sync(full, keep);
-                if(keep)
-                {
-                    const int pos = count + __popc(m & ((1u << lane) - 1u));
-                    if(pos < cap) {t.nbr[nbr_pos(pos, s, np, t.tpp, cap, t.slot_major)] = q;}
-                }
-                count += __popc(m);
-            }
-            if(lane == 0)
-            {
-                t.nnb[s] = count < cap ? count : cap;
-                atomicMax(t.max_count, count);
-                if(count > cap) {atomicOr(&a.sys[sys].status, ST_LIST_OVERFLOW);}
-            }
-        }
-    }
-}
-
-// The same list build with LPS lanes per slot (4, 8 or 16): a warp builds 32 /
-// LPS lists at once, so that short candidate sequences (a few partners per
-// stencil) do not leave most of a warp idle while it waits on memory.  A
-// group's 27 stencil ranges go through shared memory; candidate k of the
-// flattened sequence belongs to the last stencil cell whose range starts at
-// or before k; the ordered compaction within the group keeps the serial
-// walk's output order, so the lists are the same word for word.
+// every group of LPS lanes of the grid takes the next (chunk, slot) pair, so
+// that all of them have work even when only a few systems rebuild
 template<int LPS>
-__global__ void __launch_bounds__(TPB) k_build_list_sub(Arena a, int g, TermArrays t)
+__global__ void __launch_bounds__(TPB) k_build_list(Arena a, int g, TermArrays t)
 {
     constexpr int GROUPS = TPB / LPS;              // slot groups per block
     constexpr int WG = 32 / LPS;                   // slot groups per warp
-    constexpr int CPL = (27 + LPS - 1) / LPS;      // stencil cells per lane
-    __shared__ int c_start[GROUPS][27];
-    __shared__ int c_excl[GROUPS][28];             // exclusive prefix; [27] = total
-    __shared__ ExRow ex_rows[GROUPS];
-    const int n = t.work[0];
-    const int cap = t.cap;
-    const long long np = t.np;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int grp = threadIdx.x / LPS, gl = threadIdx.x % LPS;
-    const unsigned full = 0xffffffffu;
-    const unsigned gmask = ((LPS == 32) ? full : ((1u << LPS) - 1u)) << (lane - gl);
-    const long long nwork = (long long)n * CHUNK;
+    __shared__ BuildShared<LPS, TPB> sh;
+    const long long nwork = (long long)t.work[0] * CHUNK;
     const long long stride = (long long)gridDim.x * GROUPS;
     // warp-uniform loop over rounds; group (lane / LPS) of the warp takes item base + lane / LPS
-    for(long long base = (long long)blockIdx.x * GROUPS + warp * WG; base < nwork; base += stride)
+    for(long long base = (long long)blockIdx.x * GROUPS + (threadIdx.x >> 5) * WG; base < nwork; base += stride)
     {
-        const long long item = base + lane / LPS;
+        const long long item = base + (threadIdx.x & 31) / LPS;
         bool valid = item < nwork;
         int s = 0, sys = 0;
         if(valid)
@@ -459,130 +251,7 @@ __global__ void __launch_bounds__(TPB) k_build_list_sub(Arena a, int g, TermArra
             sys = w.x;
             valid = s < w.z;
         }
-        const SysDev& S = a.sys[sys];
-        const GlobalParams& G = S.g[g];
-        const bool periodic = S.boundary == B_PERIODIC;
-        const int dx_ = G.dims[0], dy_ = G.dims[1], dz_ = G.dims[2];
-        const bool wrap = periodic || G.hashed;
-        const double rl2 = G.rl2;
-        int i = 0;
-        bool lead_i = false;
-        double4 ri = make_double4(0.0, 0.0, 0.0, 0.0);
-        if(valid)
-        {
-            i = t.slot_particle[s];
-            lead_i = t.slot_lead[s] != 0;
-            ri = t.slot_pd[s];
-            stage_ex_row(a, g, i, gl, LPS, ex_rows[grp]);
-            const int cx = cell_coord(ri.x, G, 0);
-            const int cy = cell_coord(ri.y, G, 1);
-            const int cz = cell_coord(ri.z, G, 2);
-            for(int k = gl * CPL; k < gl * CPL + CPL && k < 27; ++k)   // this lane's block of stencil cells
-            {
-                int x = cx + k % 3 - 1, y = cy + (k / 3) % 3 - 1, z = cz + k / 9 - 1;
-                bool inside = true;
-                if(wrap)
-                {
-                    x = x < 0 ? x + dx_ : (x >= dx_ ? x - dx_ : x);
-                    y = y < 0 ? y + dy_ : (y >= dy_ ? y - dy_ : y);
-                    z = z < 0 ? z + dz_ : (z >= dz_ ? z - dz_ : z);
-                }
-                else if(x < 0 || y < 0 || z < 0 || x >= dx_ || y >= dy_ || z >= dz_) {inside = false;}
-                int cs = 0, cc = 0;
-                if(inside)
-                {
-                    const int cell = G.cell_off + x + dx_ * (y + dy_ * z);
-                    cs = t.cell_start[cell];
-                    cc = t.cell_count[cell];
-                    if(t.half) {clip_half(cs, cc, s);}
-                }
-                c_start[grp][k] = cs;
-                c_excl[grp][k] = cc;
-            }
-        }
-        __syncwarp();
-        // exclusive prefix of the 27 counts: within each lane's block, then
-        // across the group's lanes with shuffles
-        {
-            int cnt[CPL];
-            int sum = 0;
-#pragma unroll
-            for(int j = 0; j < CPL; ++j)
-            {
-                const int k = gl * CPL + j;
-                cnt[j] = (valid && k < 27) ? c_excl[grp][k] : 0;
-                sum += cnt[j];
-            }
-            int incl = sum;
-#pragma unroll
-            for(int o = 1; o < LPS; o <<= 1)
-            {
-                const int y = __shfl_up_sync(full, incl, o, LPS);
-                if(gl >= o) {incl += y;}
-            }
-            int run = incl - sum;
-#pragma unroll
-            for(int j = 0; j < CPL; ++j)
-            {
-                const int k = gl * CPL + j;
-                if(valid && k < 27) {c_excl[grp][k] = run;}
-                run += cnt[j];
-            }
-            if(valid && gl == LPS - 1) {c_excl[grp][27] = incl;}
-        }
-        __syncwarp();
-        const int total = valid ? c_excl[grp][27] : 0;
-        int tmax = total;
-#pragma unroll
-        for(int o = LPS; o < 32; o <<= 1) {tmax = max(tmax, __shfl_xor_sync(full, tmax, o));}
-        int count = 0;
-        int lo = 0;         // the last stencil cell whose range starts at or before k: k only grows, so
-                            // the lane walks forward from its previous cell
-        for(int b = 0; b < tmax; b += LPS)
-        {
-            const int k = b + gl;
-            bool keep = false;
-            int q = 0;
-            if(k < total)
-            {
-                while(lo < 26 && c_excl[grp][lo + 1] <= k) {++lo;}
-                q = c_start[grp][lo] + (k - c_excl[grp][lo]);
-                if(q != s)
-                {
-                    const double4 rj = t.slot_pd[q];
-                    double ddx = __dsub_rn(rj.x, ri.x);
-                    double ddy = __dsub_rn(rj.y, ri.y);
-                    double ddz = __dsub_rn(rj.z, ri.z);
-                    if(periodic)
-                    {
-                        ddx = min_image(ddx, S.halfw[0], S.width[0]);
-                        ddy = min_image(ddy, S.halfw[1], S.width[1]);
-                        ddz = min_image(ddz, S.halfw[2], S.width[2]);
-                    }
-                    const double l2 = __dadd_rn(__dadd_rn(__dmul_rn(ddx, ddx), __dmul_rn(ddy, ddy)), __dmul_rn(ddz, ddz));
-                    if(l2 < rl2)
-                    {
-                        const int j = t.slot_particle[q];
-                        const bool lead_lo = (i < j) ? lead_i : (t.slot_lead[q] != 0);
-                        keep = lead_lo && !excluded_staged(a, g, G.ignore_mol, ex_rows[grp], i, j);
-                    }
-                }
-            }
-            const unsigned m = __ballot_sync(full, keep) & gmask;
-            if(keep)
-            {
-                const int pos = count + __popc(m & ((1u << lane) - 1u));
-                if(pos < cap) {t.nbr[nbr_pos(pos, s, np, t.tpp, cap, t.slot_major)] = q;}
-            }
-            count += __popc(m);
-        }
-        if(valid && gl == 0)
-        {
-            t.nnb[s] = count < cap ? count : cap;
-            atomicMax(t.max_count, count);
-            if(count > cap) {atomicOr(&a.sys[sys].status, ST_LIST_OVERFLOW);}
-        }
-        __syncwarp();
+        build_list_group<LPS, TPB>(a, g, t, valid, sys, s, sh);
     }
 }
 
@@ -608,6 +277,15 @@ __global__ void k_scatter_param(TermArrays t, double* w)
     if(p < t.np) {w[t.part_particle[p]] = t.part_p0[p];}
 }
 
+__global__ void __launch_bounds__(TPB) k_sum_counts(TermArrays t)
+{
+    unsigned long long v = 0;
+    for(long long s = (long long)blockIdx.x * TPB + threadIdx.x; s < t.np; s += (long long)gridDim.x * TPB) {v += t.slot_part[s];}
+#pragma unroll
+    for(int o = 16; o > 0; o >>= 1) {v += __shfl_xor_sync(0xffffffffu, v, o);}
+    if((threadIdx.x & 31) == 0) {atomicAdd(t.total_count, v);}
+}
+
 inline unsigned blocks(long long n, int tpb = TPB) {return (unsigned)((n + tpb - 1) / tpb);}
 
 }  // namespace
@@ -616,6 +294,12 @@ void launch_scatter_param(const TermArrays& t, double* w, cudaStream_t s)
 {
     if(!t.on || t.np == 0) {return;}
     k_scatter_param<<<blocks(t.np), TPB, 0, s>>>(t, w);
+    note_launches(1);
+}
+
+void launch_sum_counts(const TermArrays& t, cudaStream_t s)
+{
+    k_sum_counts<<<min(blocks(t.np), (unsigned)GRID), TPB, 0, s>>>(t);
     note_launches(1);
 }
 
@@ -629,10 +313,10 @@ void launch_rebuild(const Arena& a, int g, TermArrays& t, int force_all, cudaStr
     k_cells_scatter<<<GRID, TPB, 0, s>>>(t, t.slot_particle);
     k_cells_sort  <<<GRID, TPB, 0, s>>>(t, t.slot_particle);
     k_slots_setup <<<GRID, TPB, 0, s>>>(a, t);
-    if(t.build_lanes == 4)       {k_build_list_sub<4> <<<GRID, TPB, 0, s>>>(a, g, t);}
-    else if(t.build_lanes == 8)  {k_build_list_sub<8> <<<GRID, TPB, 0, s>>>(a, g, t);}
-    else if(t.build_lanes == 16) {k_build_list_sub<16><<<GRID, TPB, 0, s>>>(a, g, t);}
-    else                         {k_build_list        <<<GRID, TPB, 0, s>>>(a, g, t);}
+    if(t.build_lanes == 4)       {k_build_list<4> <<<GRID, TPB, 0, s>>>(a, g, t);}
+    else if(t.build_lanes == 8)  {k_build_list<8> <<<GRID, TPB, 0, s>>>(a, g, t);}
+    else if(t.build_lanes == 16) {k_build_list<16><<<GRID, TPB, 0, s>>>(a, g, t);}
+    else                         {k_build_list<32><<<GRID, TPB, 0, s>>>(a, g, t);}
     k_rebuild_done<<<blocks(a.nsys, 128), 128, 0, s>>>(a, g, t, force_all);
     note_launches(9);
 }

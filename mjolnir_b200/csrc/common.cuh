@@ -70,6 +70,7 @@ struct GlobalParams {       // per system, per global term
     int    slot_off;        // first slot of this system (participant offset)
     int    nslot;
     int    ignore_mol;      // IgnoreMol
+    int    last;            // particle of the last participant, which leads no list
     int    rebuild;         // set by the margin kernel, cleared after a rebuild
     int    rebuilds;        // rebuild counter
     int    kind;            // the term's potential (ExvKind for the first, LjKind for the third)
@@ -77,10 +78,11 @@ struct GlobalParams {       // per system, per global term
     int    on;
 };
 
-struct SysDev {
+struct alignas(16) SysDev {
     long long off, n;       // particle range in the arena
     int    boundary, integrator;
     double lower[3], upper[3], width[3], halfw[3];
+    int    halfw_hi;        // high word of the smallest halfw; 0x7fffffff without a periodic box
     unsigned long long seed;
     unsigned long long step;
     unsigned long long max_disp2;   // bits of a non-negative double (atomicMax)
@@ -113,6 +115,19 @@ __device__ __forceinline__ double min_image(double d, double halfw, double width
     if(d < -halfw)       {d = __dadd_rn(d, width);}
     else if(d >= halfw)  {d = __dsub_rn(d, width);}
     return d;
+}
+
+// Whether min_image may change a component of a displacement: some |d| is not
+// below the smallest half width, compared by the high words of the doubles
+// (integer pipe; never false where an image is due).  Most pairs lie within
+// half a box as they are, and without a periodic box (halfw_hi = 0x7fffffff)
+// none needs an image, so one test takes the place of two FP64 comparisons and
+// two selections per component.
+__device__ __forceinline__ bool image_needed(double dx, double dy, double dz, int halfw_hi)
+{
+    const int m = max(max(__double2hiint(dx) & 0x7fffffff, __double2hiint(dy) & 0x7fffffff),
+                      __double2hiint(dz) & 0x7fffffff);
+    return m >= halfw_hi;
 }
 
 // ------------------------------------------------------- Philox4x32-10

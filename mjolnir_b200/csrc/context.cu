@@ -131,9 +131,9 @@ struct HostSystem {
 };
 
 struct TermDev {
-    DevBuf part_particle, part_p0, part_p1, part_lead, part_sys, part_cell;
+    DevBuf part_particle, part_p0, part_p1, part_sys, part_cell;
     DevBuf cell_count, cell_start, cell_fill, work, part_chunks, cell_chunks, flagged;
-    DevBuf slot_part, slot_particle, slot_lead, slot_sys, slot_pd, slot_p1, slot_of, slot_w;
+    DevBuf slot_part, slot_particle, slot_sys, slot_pd, slot_p1, slot_of, slot_w;
     DevBuf nnb, nbr, max_count, any_rebuild;
     DevBuf ex_start, ex_idx;
     int cap_alloc = 0;           // capacity the nbr buffer was sized for
@@ -215,9 +215,9 @@ int64_t device_bytes(const mjg_context* c)
     for(auto* x : bufs) {b += (int64_t)x->cap;}
     for(const auto& t : c->term)
     {
-        const DevBuf* tb[] = {&t.part_particle, &t.part_p0, &t.part_p1, &t.part_lead, &t.part_sys,
+        const DevBuf* tb[] = {&t.part_particle, &t.part_p0, &t.part_p1, &t.part_sys,
                               &t.part_cell, &t.cell_count, &t.cell_start, &t.cell_fill,
-                              &t.work, &t.part_chunks, &t.cell_chunks, &t.flagged, &t.slot_part, &t.slot_particle, &t.slot_lead,
+                              &t.work, &t.part_chunks, &t.cell_chunks, &t.flagged, &t.slot_part, &t.slot_particle,
                               &t.slot_sys, &t.slot_pd, &t.slot_p1, &t.slot_of, &t.slot_w, &t.nnb, &t.nbr, &t.max_count,
                               &t.any_rebuild, &t.ex_start, &t.ex_idx};
         for(auto* x : tb) {b += (int64_t)x->cap;}
@@ -412,12 +412,14 @@ int list_capacity(int max_count) {return ((max_count + max_count / 4 + 16) + 31)
 // threads per slot of the pair kernel from the longest list, widened for
 // arenas with few slots until the launch fills the GPU (about 148 SMs x 1,024
 // threads; a small system otherwise leaves most SMs idle and each thread
-// walks a long chain of dependent loads); refined by the autotuner through
-// mjg_set_threads_per_particle
-int default_tpp(int max_count, long long slots)
+// walks a long chain of dependent loads), but not past the mean length: more
+// threads than a list has partners only add warps that wait (10,000-bead melt
+// alone, ExcludedVolume lists of about 5: 4 threads instead of 16).  Refined by
+// the autotuner through mjg_set_threads_per_particle.
+int default_tpp(int max_count, double mean_count, long long slots)
 {
     int tpp = max_count >= 192 ? 8 : (max_count >= 48 ? 4 : (max_count >= 12 ? 2 : 1));
-    while(tpp < 32 && tpp < max_count && slots * tpp < 148LL * 1024) {tpp *= 2;}
+    while(tpp < 32 && 2 * tpp <= mean_count && slots * tpp < 148LL * 1024) {tpp *= 2;}
     return tpp;
 }
 
@@ -436,6 +438,18 @@ void alloc_lists(mjg_context* c, int g, int cap)
     T.t.cap = cap;
     T.cap_alloc = cap;
     release_graph(c);
+}
+
+// mean list length of term g at the last forced build, before any cut at the capacity
+double mean_count(mjg_context* c, int g)
+{
+    const TermArrays& t = c->term[g].t;
+    unsigned long long total = 0;
+    CK(cudaMemsetAsync(t.total_count, 0, sizeof(total), c->stream));
+    launch_sum_counts(t, c->stream);
+    CK(cudaMemcpyAsync(&total, t.total_count, sizeof(total), cudaMemcpyDeviceToHost, c->stream));
+    CK(cudaStreamSynchronize(c->stream));
+    return (double)total / (double)t.np;
 }
 
 // forced rebuild of every list; grows capacities until nothing overflows
@@ -461,7 +475,7 @@ void rebuild_all(mjg_context* c)
         if(!T.t.on || T.t.np == 0) {continue;}
         for(int k = 0; k < 3 && mx[g] > T.t.cap; ++k)
         {
-            if(!T.tpp_fixed) {T.t.tpp = default_tpp(mx[g], T.t.np);}
+            if(!T.tpp_fixed) {T.t.tpp = default_tpp(mx[g], mean_count(c, g), T.t.np);}
             alloc_lists(c, g, list_capacity(mx[g]));
             attempt(g);
             CK(cudaStreamSynchronize(c->stream));
@@ -763,6 +777,14 @@ void make_sysdev(const HostSystem& s, SysDev& d)
         d.width[x] = s.upper[x] - s.lower[x];
         d.halfw[x] = d.width[x] / 2;
     }
+    d.halfw_hi = 0x7fffffff;
+    if(s.boundary == B_PERIODIC)
+    {
+        const double w = std::min(d.halfw[0], std::min(d.halfw[1], d.halfw[2]));
+        long long bits;
+        std::memcpy(&bits, &w, sizeof bits);
+        d.halfw_hi = (int)(bits >> 32);
+    }
     d.seed = s.seed;
     d.step = s.step;
     d.frozen = s.frozen ? 1 : 0;
@@ -893,8 +915,7 @@ void commit(mjg_context* c)
     Carver cv;
     const auto c_pos = cv.add<double4>(n_tot), c_vel = cv.add<double4>(n_tot), c_coef = cv.add<double4>(n_tot);
     const auto c_psys = cv.add<int>(n_tot), c_mol = cv.add<int>(n_tot);
-    Carver::Item c_exs[NGLOBAL], c_exi[NGLOBAL], c_pp[NGLOBAL], c_ps[NGLOBAL], c_p0[NGLOBAL], c_p1[NGLOBAL],
-                 c_pl[NGLOBAL];
+    Carver::Item c_exs[NGLOBAL], c_exi[NGLOBAL], c_pp[NGLOBAL], c_ps[NGLOBAL], c_p0[NGLOBAL], c_p1[NGLOBAL];
     for(int g = 0; g < NGLOBAL; ++g)
     {
         c_exs[g] = cv.add<long long>(n_tot + 1);
@@ -903,7 +924,6 @@ void commit(mjg_context* c)
         c_ps[g] = cv.add<int>(np_tot[g]);
         c_p0[g] = cv.add<double>(np_tot[g]);
         c_p1[g] = cv.add<double>(np_tot[g]);
-        c_pl[g] = cv.add<unsigned char>(np_tot[g]);
     }
     const auto c_bidx = cv.add<int>(2 * nb), c_bk = cv.add<double>(nb), c_bv0 = cv.add<double>(nb),
                c_bsys = cv.add<int>(nb), c_bkv = cv.add<float2>(nb);
@@ -1005,8 +1025,8 @@ void commit(mjg_context* c)
             const HostGlobal& H = s.g[g];
             int* pp = (int*)at(c_pp[g]); int* ps = (int*)at(c_ps[g]);
             double* p0 = (double*)at(c_p0[g]); double* p1 = (double*)at(c_p1[g]);
-            unsigned char* pl = (unsigned char*)at(c_pl[g]);
             const int64_t np = G.nslot;
+            hs[k].g[g].last = np > 0 ? (int)(off + H.idx[np - 1]) : -1;
             for(int64_t q = 0; q < np; ++q)
             {
                 const int64_t x = G.slot_off + q;
@@ -1014,7 +1034,6 @@ void commit(mjg_context* c)
                 ps[x] = (int)k;
                 p0[x] = H.p0[q];
                 p1[x] = H.p1.empty() ? 0.0 : H.p1[q];
-                pl[x] = q + 1 < np ? 1 : 0;
             }
         }
         for(int64_t t = 0; t < s.bond.m(); ++t)
@@ -1145,9 +1164,9 @@ void commit(mjg_context* c)
         t.ncell = (int)ncell[g];
         if(!t.on)
         {
-            DevBuf* bufs[] = {&T.part_particle, &T.part_p0, &T.part_p1, &T.part_lead, &T.part_sys,
+            DevBuf* bufs[] = {&T.part_particle, &T.part_p0, &T.part_p1, &T.part_sys,
                               &T.part_cell, &T.cell_count, &T.cell_start, &T.cell_fill,
-                              &T.work, &T.part_chunks, &T.cell_chunks, &T.flagged, &T.slot_part, &T.slot_particle, &T.slot_lead,
+                              &T.work, &T.part_chunks, &T.cell_chunks, &T.flagged, &T.slot_part, &T.slot_particle,
                               &T.slot_sys, &T.slot_pd, &T.slot_p1, &T.slot_of, &T.slot_w, &T.nnb, &T.nbr,
                               &T.max_count, &T.any_rebuild};
             for(auto* b : bufs) {b->release();}
@@ -1157,7 +1176,6 @@ void commit(mjg_context* c)
         put(T.part_particle, c_pp[g]);
         put(T.part_p0, c_p0[g]);
         put(T.part_p1, c_p1[g]);
-        put(T.part_lead, c_pl[g]);
         put(T.part_sys, c_ps[g]);
         T.part_cell.ensure(sizeof(int) * np);
         T.cell_count.ensure(sizeof(int) * t.ncell);
@@ -1179,7 +1197,6 @@ void commit(mjg_context* c)
         CK(cudaMemsetAsync(T.cell_fill.p, 0, T.cell_fill.bytes, st));
         T.slot_part.ensure(sizeof(int) * np);
         T.slot_particle.ensure(sizeof(int) * np);
-        T.slot_lead.ensure(np);
         T.slot_sys.ensure(sizeof(int) * np);
         T.slot_pd.ensure(sizeof(double4) * np);
         T.slot_p1.ensure(sizeof(double) * np);
@@ -1187,14 +1204,13 @@ void commit(mjg_context* c)
         CK(cudaMemsetAsync(T.slot_of.p, 0xff, T.slot_of.bytes, st));      // -1: no slot
         T.slot_w.ensure(sizeof(double) * (size_t)std::max<long long>(n_tot, 1));
         T.nnb.ensure(sizeof(int) * np);
-        T.max_count.ensure(sizeof(int));
+        T.max_count.ensure(2 * sizeof(unsigned long long));      // longest list; sum of the lengths
         T.any_rebuild.ensure(sizeof(int));
         CK(cudaMemsetAsync(T.any_rebuild.p, 0, sizeof(int), st));
         CK(cudaMemsetAsync(T.nnb.p, 0, T.nnb.bytes, st));
         t.part_particle = T.part_particle.as<int>();
         t.part_p0 = T.part_p0.as<double>();
         t.part_p1 = T.part_p1.as<double>();     // LJ-family epsilon, HardCore core radius
-        t.part_lead = T.part_lead.as<unsigned char>();
         t.part_sys = T.part_sys.as<int>();
         t.part_cell = T.part_cell.as<int>();
         t.cell_count = T.cell_count.as<int>();
@@ -1206,7 +1222,6 @@ void commit(mjg_context* c)
         t.flagged = T.flagged.as<int>();
         t.slot_part = T.slot_part.as<int>();
         t.slot_particle = T.slot_particle.as<int>();
-        t.slot_lead = T.slot_lead.as<unsigned char>();
         t.slot_sys = T.slot_sys.as<int>();
         t.slot_pd = T.slot_pd.as<double4>();
         t.slot_p1 = T.slot_p1.as<double>();
@@ -1217,6 +1232,7 @@ void commit(mjg_context* c)
         launch_scatter_param(t, T.slot_w.as<double>(), st);
         t.nnb = T.nnb.as<int>();
         t.max_count = T.max_count.as<int>();
+        t.total_count = T.max_count.as<unsigned long long>() + 1;
         t.any_rebuild = T.any_rebuild.as<int>();
         t.tpp = T.tpp_fixed ? T.tpp_choice : 1;
         t.unroll = T.unroll_choice;
@@ -1517,9 +1533,9 @@ void mjg_context_destroy(mjg_context* c)
     release_graph(c);
     for(auto& t : c->term)
     {
-        DevBuf* bufs[] = {&t.part_particle, &t.part_p0, &t.part_p1, &t.part_lead, &t.part_sys,
+        DevBuf* bufs[] = {&t.part_particle, &t.part_p0, &t.part_p1, &t.part_sys,
                           &t.part_cell, &t.cell_count, &t.cell_start, &t.cell_fill, &t.work, &t.part_chunks, &t.cell_chunks, &t.flagged,
-                          &t.slot_part, &t.slot_particle, &t.slot_lead, &t.slot_sys, &t.slot_pd,
+                          &t.slot_part, &t.slot_particle, &t.slot_sys, &t.slot_pd,
                           &t.slot_p1, &t.slot_of, &t.slot_w, &t.nnb, &t.nbr, &t.max_count, &t.any_rebuild, &t.ex_start,
                           &t.ex_idx};
         for(auto* b : bufs) {b->release();}

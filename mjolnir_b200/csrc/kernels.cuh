@@ -61,7 +61,6 @@ struct TermArrays {
     const int* part_particle;   // [np] global particle index
     const double* part_p0;      // [np] radius / charge / sigma
     const double* part_p1;      // [np] LJ epsilon
-    const unsigned char* part_lead; // [np] leading participant
     const int* part_sys;        // [np]
     int*       part_cell;       // [np]
     int*       cell_count;      // [ncell]
@@ -71,9 +70,8 @@ struct TermArrays {
     int4*      part_chunks;     // rebuild work: participant chunks {sys, begin, end}
     int4*      cell_chunks;     // rebuild work: cell chunks
     int*       flagged;         // [nsys] systems rebuilding this step
-    int*       slot_part;       // [np] participant of slot (cell order)
+    int*       slot_part;       // [np] scratch of the rebuild: participants in cell order, then list lengths
     int*       slot_particle;   // [np] global particle of slot
-    unsigned char* slot_lead;   // [np]
     int*       slot_sys;        // [np]
     double4*   slot_pd;         // [np] x, y, z, p0 (kept current by the integrator)
     int*       slot_of;         // [n] slot of each particle of the arena, -1 if none
@@ -81,6 +79,7 @@ struct TermArrays {
     int*       nnb;             // [np] partners per slot
     int*       nbr;             // [cap * np] column-major
     int*       max_count;       // [1] largest list seen at the last build
+    unsigned long long* total_count;   // [1] launch_sum_counts
     int*       any_rebuild;     // [1]
 };
 
@@ -110,6 +109,8 @@ void launch_integrate_last(const Arena& a, cudaStream_t s);
 void launch_zero_force(const Arena& a, cudaStream_t s);
 
 void launch_rebuild(const Arena& a, int gterm, TermArrays& t, int force_all, cudaStream_t s);
+// total_count = sum of the list lengths (before any cut at the capacity) of the last build of every system
+void launch_sum_counts(const TermArrays& t, cudaStream_t s);
 // w[particle] = the term's parameter of each participant (radius, charge, sigma)
 void launch_scatter_param(const TermArrays& t, double* w, cudaStream_t s);
 // slot coordinates of a term's participants (before its force launch)
