@@ -28,6 +28,7 @@ enum : int {
     ST_LIST_OVERFLOW  = 1,   // a neighbour list exceeded its capacity
     ST_FIXED_OVERFLOW = 2,   // a force left the fixed-point range
     ST_NONFINITE      = 4,   // a non-finite force or position
+    ST_BARRIER        = 8,   // a grid barrier of the multi-step kernel ran out of time (system 0)
 };
 
 // Fixed-point forces: value = integer * 2^-FX_SHIFT.  Conversion uses the

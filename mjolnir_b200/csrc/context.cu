@@ -175,6 +175,8 @@ struct mjg_context {
     mjg::DevBuf d_accel;                        // UnderdampedLangevin accelerations
     mjg::DevBuf b_sys, b_pos, b_vel, b_force, b_accel;   // rollback copies
     mjg::DevBuf d_force_scratch;
+    mjg::DevBuf d_run;                      // multi-step kernel: barrier word, displacements
+    int sms = 0;                            // SMs of the device
     double* h_pinned = nullptr;             // page-locked host staging (state, forces)
     size_t h_pinned_bytes = 0;
     void* h_pack = nullptr;                 // page-locked packing buffer of commit
@@ -207,7 +209,7 @@ int64_t device_bytes(const mjg_context* c)
     const DevBuf* bufs[] = {&c->d_sys, &c->d_pos, &c->d_vel, &c->d_force, &c->d_coef, &c->d_psys,
                             &c->d_staging, &c->d_mol, &c->b_sys, &c->b_pos, &c->b_vel, &c->b_force,
                             &c->d_accel, &c->b_accel,
-                            &c->d_force_scratch, &c->l_bond_idx, &c->l_bond_k, &c->l_bond_v0,
+                            &c->d_force_scratch, &c->d_run, &c->l_bond_idx, &c->l_bond_k, &c->l_bond_v0,
                             &c->l_bond_sys, &c->l_angle_idx, &c->l_angle_k, &c->l_angle_v0,
                             &c->l_angle_sys, &c->l_dihd_idx, &c->l_dihd_k, &c->l_dihd_n,
                             &c->l_dihd_v0, &c->l_dihd_sys, &c->l_win_bond, &c->l_win_angle,
@@ -1104,6 +1106,8 @@ void commit(mjg_context* c)
     put(c->d_mol, c_mol);
     c->d_force.ensure(32 * (size_t)std::max<long long>(n_tot, 1));
     c->d_force_scratch.ensure(32 * (size_t)std::max<long long>(n_tot, 1));
+    c->d_run.ensure(256 + sizeof(unsigned long long) * 2 * RUN_MAX_SYSTEMS);
+    CK(cudaMemsetAsync(c->d_run.p, 0, c->d_run.bytes, st));
     // the per-particle auxiliary array: UnderdampedLangevin accelerations,
     // G-JF coefficients
     bool any_underdamped = false, any_gjf = false;
@@ -1398,6 +1402,11 @@ void check_status(mjg_context* c, bool& overflow)
     // a list overflow is handled (rolled back) before anything else is checked
     for(const auto& d : c->h_sys) {if(d.status & ST_LIST_OVERFLOW) {overflow = true;}}
     if(overflow) {return;}
+    if(!c->h_sys.empty() && (c->h_sys[0].status & ST_BARRIER))
+    {
+        cudaMemsetAsync(c->d_run.p, 0, c->d_run.bytes, c->stream);   // the arrival word stopped half-way
+        throw Error(MJG_ECUDA, "a grid barrier of the multi-step kernel ran out of time");
+    }
     for(size_t k = 0; k < c->h_sys.size(); ++k)
     {
         const int st = c->h_sys[k].status;
@@ -1412,6 +1421,20 @@ void check_status(mjg_context* c, bool& overflow)
                         ": non-finite displacement (the system blew up)");
         }
     }
+}
+
+// Arenas whose chunks run in the multi-step kernel: there a step's launches and
+// gaps cost more than its work.  Measured (graph of launches / multi-step, us
+// per step): 200 beads 23 / 9.4, 4,096 Lennard-Jones 33 / 17.6, 10,000-bead
+// melt 31 / 14.8, 40 melts of 115,000 beads in all 73 / 71, 262,144-bead fluid
+// 440 / 415 (FP64, untuned shapes), 1,048,576-bead fluid 1150 / 1210 (tuned
+// shapes, which the multi-step kernel has no form of); the line lies where the
+// two meet.
+constexpr long long RUN_MAX_PARTICLES = 131072;
+constexpr int64_t RUN_STEPS = 1024;             // steps per launch
+bool run_fits(const mjg_context* c)
+{
+    return c->arena.n > 0 && c->arena.n <= RUN_MAX_PARTICLES && c->arena.nsys <= RUN_MAX_SYSTEMS;
 }
 
 void run_steps(mjg_context* c, int64_t nsteps)
@@ -1433,7 +1456,23 @@ void run_steps(mjg_context* c, int64_t nsteps)
         }
         // step 1 of the chunk, then steps 2..n with the previous closing
         // half-kick fused into their first pass, then the last closing kick
-        if(c->graphs)
+        if(c->graphs && run_fits(c))
+        {
+            RunArgs r{};
+            r.a = c->arena;
+            for(int g = 0; g < NGLOBAL; ++g) {r.t[g] = c->term[g].t;}
+            r.l = c->local;
+            r.barrier = c->d_run.as<unsigned>();
+            r.disp2 = reinterpret_cast<unsigned long long*>(c->d_run.as<char>() + 256);
+            for(int64_t k = 0; k < nsteps; k += RUN_STEPS)
+            {
+                r.nsteps = (int)std::min<int64_t>(RUN_STEPS, nsteps - k);
+                r.kick = k > 0 ? 1 : 0;
+                r.close = k + r.nsteps == nsteps ? 1 : 0;
+                CK(launch_run(r, c->sms, st));
+            }
+        }
+        else if(c->graphs)
         {
             if(c->graph_dirty || !c->graph_exec) {capture_graph(c);}
             CK(cudaGraphLaunch(c->graph_exec, st));
@@ -1447,7 +1486,7 @@ void run_steps(mjg_context* c, int64_t nsteps)
         {
             for(int64_t k = 0; k < nsteps; ++k) {enqueue_step_body(c, k > 0, false);}
         }
-        launch_integrate_last(c->arena, st);
+        if(!(c->graphs && run_fits(c))) {launch_integrate_last(c->arena, st);}
         CK(cudaGetLastError());
         download_sys(c);
         bool overflow = false;
@@ -1504,6 +1543,7 @@ int mjg_context_create(int device, int precision, mjg_context** out)
     c->device = device;
     c->precision = precision;
     bool ok = cudaSetDevice(device) == cudaSuccess &&
+              cudaDeviceGetAttribute(&c->sms, cudaDevAttrMultiProcessorCount, device) == cudaSuccess &&
               cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) == cudaSuccess &&
               cudaEventCreateWithFlags(&c->ev_fork, cudaEventDisableTiming) == cudaSuccess;
     for(int b = 0; ok && b <= mjg::NGLOBAL; ++b)

@@ -153,6 +153,22 @@ void launch_set_noise(const Arena& a, const double* noise, long long first, long
 void launch_set_force(const Arena& a, const double* src, long long first, long long count,
                       cudaStream_t s);
 
+// Many steps of a small arena in one launch (run.cu).
+constexpr int RUN_MAX_SYSTEMS = 64;
+constexpr int RUN_CLUSTER_MAX = 8;   // blocks up to which the launch is one cluster (the portable size)
+struct RunArgs {
+    Arena a;
+    TermArrays t[NGLOBAL];
+    LocalArrays l;
+    unsigned* barrier;               // arrival word of the grid barrier (zero before its first use)
+    unsigned long long* disp2;       // [2 nsys] largest squared displacements, zero between launches
+    int nsteps;
+    int kick;                        // open with the closing half of the step before this launch
+    int close;                       // end with the closing half of the last step
+    int cluster;                     // set by the launch: the grid is one cluster
+};
+cudaError_t launch_run(RunArgs r, int sms, cudaStream_t s);
+
 // kernel launch accounting (every wrapper reports what it enqueued)
 void note_launches(int k);
 

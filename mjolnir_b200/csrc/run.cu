@@ -1,0 +1,592 @@
+// Many MD steps in one launch, for arenas small enough that a step's launches
+// and the gaps between them, not its work, set its time.
+//
+// One resident grid (one block of 1,024 threads per SM at most, launched
+// cooperatively) walks the step's phases itself -- integrator pass, margin
+// bookkeeping, list rebuilds of the systems that need them, forces -- with a
+// barrier between phases, so a step without a rebuild costs two barriers
+// instead of a chain of dependent graph nodes.  What bounds it is the latency
+// of each phase's chain of dependent loads plus the barriers (about a
+// microsecond each over the whole GPU, less within one cluster), so the work
+// of a phase is spread warp by warp over every SM: consecutive warp items go
+// to different blocks.  The arithmetic is that of the step's launches
+// (advance_particle, PairEval, the bonded formulas, the list builds), so in
+// the mixed form, whose force sums are exact, a chunk gives the same bits
+// either way.
+//
+// Measured (graph of launches / this kernel, us per step): 200-bead chain 23 /
+// 9.4, 4,096-particle Lennard-Jones fluid 33 / 17.6 mixed and 32 / 16.9 FP64,
+// 2,997-bead melt 24.6 / 12.1, 10,000-bead melt FP64 31 / 14.8.  Of the
+// Lennard-Jones fluid's 17.6 the integrator pass takes 1.8, its barrier 1.3,
+// the margins 0.8, the forces 5.7, the second barrier with the noise drawn
+// meanwhile 1.8, and a twelfth of a rebuild 3.1.
+//
+// Every load here is a plain one: lists, slot coordinates and cells are
+// rewritten during the launch, which the read-only path must not see.
+#include "integrate.cuh"
+#include "list_build.cuh"
+#include "local_terms.cuh"
+#include "pair_eval.cuh"
+
+#include <algorithm>
+
+namespace mjg {
+
+namespace {
+
+constexpr int RT = 1024;                 // threads per block
+constexpr int RUN_BATCH = 2;             // partners a thread requests together
+constexpr int CELL_CHUNK = RT;           // cells per scan item
+
+using ull = unsigned long long;
+
+// ------------------------------------------------------------------ barrier
+// All blocks of the grid.  A launch that fits one cluster uses the cluster's
+// hardware barrier.  Otherwise one word counts arrivals: every block adds 1,
+// block 0 adds what takes the sum to the next multiple of 2^31, and a waiting
+// block watches the top bit flip, so the word needs no reset between barriers
+// or launches.  The wait is bounded in time (BARRIER_CYCLES, about a second): a
+// block that gives up raises ST_BARRIER, and every block returns at its next
+// barrier.
+constexpr long long BARRIER_CYCLES = 2LL << 30;
+
+// The last warp's first lane arrives and polls: the first warps hold the
+// particles (Grid::warp), whose noise is drawn meanwhile.
+constexpr int POLLER = RT - 32;
+struct Barrier {
+    unsigned* word;
+    int* status;
+    bool cluster;
+    unsigned old;
+    __device__ __forceinline__ void arrive()
+    {
+        if(cluster)
+        {
+            asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+            return;
+        }
+        __syncthreads();
+        if(threadIdx.x == POLLER)
+        {
+            const unsigned add = blockIdx.x == 0 ? 0x80000000u - (gridDim.x - 1) : 1u;
+            asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], %2;" : "=r"(old) : "l"(word), "r"(add) : "memory");
+        }
+    }
+    __device__ __forceinline__ bool wait()
+    {
+        if(cluster)
+        {
+            asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+            return true;
+        }
+        int ok = 1;
+        if(threadIdx.x == POLLER)
+        {
+            unsigned now;
+            const long long t0 = clock64();
+            for(;;)
+            {
+                asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(now) : "l"(word) : "memory");
+                if((old ^ now) & 0x80000000u) {break;}
+                if(clock64() - t0 > BARRIER_CYCLES) {atomicOr(status, ST_BARRIER); ok = 0; break;}
+            }
+        }
+        return __syncthreads_and(ok) != 0;
+    }
+    __device__ __forceinline__ bool sync() {arrive(); return wait();}
+};
+
+// ------------------------------------------------- bonded forces, one by one
+// Each term adds its forces to the particles directly: in a small arena the
+// block-wide window of the bonded launch would only lengthen the chain.
+template<int PREC>
+struct DirectAdd {
+    __device__ __forceinline__ void add(void* force, int i, double fx, double fy, double fz)
+    {
+        Window<PREC>::global_add(force, i, fx, fy, fz);
+    }
+};
+
+__device__ __forceinline__ void add_force(void* force, long long i, const Acc<P_MIXED>& acc) {acc.store(force, i);}
+// The plain form adds with FP64 atomics here: the terms of one particle land
+// in any order (the launches of a step add them one term after the other).
+__device__ __forceinline__ void add_force(void* force, long long i, const Acc<P_FP64>& acc)
+{
+    double* f = reinterpret_cast<double*>(static_cast<double4*>(force) + i);
+    atomicAdd(f + 0, acc.x); atomicAdd(f + 1, acc.y); atomicAdd(f + 2, acc.z);
+}
+
+// ------------------------------------------------------------------ rebuild
+
+// The launch works on its own copy of the system records in shared memory
+// (dynamic; the arena's pointer is replaced by it), read by every phase without
+// a trip to L2; the remaining skins are kept there by every block for itself.
+struct Shared {
+    int chunk_off[RUN_MAX_SYSTEMS][NGLOBAL];     // first chunk sum of each system
+    int rebuilds[RUN_MAX_SYSTEMS][NGLOBAL];
+    ull flag[NGLOBAL];                           // systems to rebuild, a bit each
+    int scan[32];
+    int carry;
+    union {
+        BuildShared<8, RT> narrow;
+        BuildShared<32, RT> wide;
+    };
+};
+
+// element k of the concatenation of the flagged systems' ranges (n(s)
+// elements each): the system and the index in its range
+template<class N>
+__device__ __forceinline__ bool locate(ull mask, int& k, int& s, N&& n)
+{
+    for(; mask; mask &= mask - 1)
+    {
+        s = __ffsll((long long)mask) - 1;
+        const int c = n(s);
+        if(k < c) {return true;}
+        k -= c;
+    }
+    return false;
+}
+
+struct Grid {
+    int nwarp, warp;             // warps of the grid; this warp, consecutive warps on different SMs
+    int nthread, thread;
+    __device__ Grid()
+    {
+        nwarp = gridDim.x * (RT / 32);
+        warp = (threadIdx.x >> 5) * gridDim.x + blockIdx.x;
+        nthread = nwarp * 32;
+        thread = warp * 32 + (threadIdx.x & 31);
+    }
+};
+
+template<int LPS>
+__device__ __forceinline__ void build(const Arena& a, int g, const TermArrays& t, ull mask, const Grid& G,
+                                      BuildShared<LPS, RT>& sh)
+{
+    constexpr int WG = 32 / LPS;             // slots per warp
+    auto nslot = [&](int s) {return a.sys[s].g[g].nslot;};
+    int s = 0;
+    for(int base = G.warp * WG;; base += G.nwarp * WG)
+    {
+        int k = base;
+        if(!locate(mask, k, s, nslot)) {break;}
+        k = base + (threadIdx.x & 31) / LPS;
+        const bool valid = locate(mask, k, s, nslot);
+        build_list_group<LPS, RT>(a, g, t, valid, s, valid ? a.sys[s].g[g].slot_off + k : 0, sh);
+    }
+}
+
+// The lists of the flagged systems of term g at the current positions.  The
+// cell counters and chunk sums are zero on entry (the force phase that follows
+// each rebuild clears them).
+template<int g>
+__device__ __forceinline__ bool rebuild(const Arena& a, const TermArrays& t, ull mask, const Grid& G, Shared& sh,
+                                        Barrier& bar)
+{
+    int* const csum = reinterpret_cast<int*>(t.cell_chunks);
+    int* const rank = t.nnb;                 // scratch until the build writes the lengths
+    auto nslot = [&](int s) {return a.sys[s].g[g].nslot;};
+    int k, s = 0;
+    // bin the participants; each takes its place within its cell
+    for(int e = G.thread;; e += G.nthread)
+    {
+        k = e;
+        if(!locate(mask, k, s, nslot)) {break;}
+        const GlobalParams& P = a.sys[s].g[g];
+        const int p = P.slot_off + k;
+        const double4 x = a.pos[t.part_particle[p]];
+        const int c = cell_coord(x.x, P, 0) + P.dims[0] * (cell_coord(x.y, P, 1) + P.dims[1] * cell_coord(x.z, P, 2));
+        t.part_cell[p] = P.cell_off + c;
+        rank[p] = atomicAdd(&t.cell_count[P.cell_off + c], 1);
+        if(P.ncell > CELL_CHUNK)                 // a single chunk's sum is not read
+        {
+            const int chunk = sh.chunk_off[s][g] + c / CELL_CHUNK;
+            const unsigned same = __match_any_sync(__activemask(), chunk);
+            if((threadIdx.x & 31) == __ffs(same) - 1) {atomicAdd(&csum[chunk], __popc(same));}
+        }
+    }
+    if(!bar.sync()) {return false;}
+    // first slot of each cell: one block per chunk of cells; the sums of the
+    // system's earlier chunks are added up by the block that needs them
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    for(int e = blockIdx.x;; e += gridDim.x)
+    {
+        k = e;
+        if(!locate(mask, k, s, [&](int x) {return (a.sys[x].g[g].ncell + CELL_CHUNK - 1) / CELL_CHUNK;})) {break;}
+        const GlobalParams& q = a.sys[s].g[g];
+        int before = 0;
+        for(int c = threadIdx.x; c < k; c += RT) {before += csum[sh.chunk_off[s][g] + c];}
+        before = __reduce_add_sync(0xffffffffu, before);
+        const int cell = k * CELL_CHUNK + threadIdx.x;
+        const int v = cell < q.ncell ? t.cell_count[q.cell_off + cell] : 0;
+        int incl = v;
+#pragma unroll
+        for(int o = 1; o < 32; o <<= 1)
+        {
+            const int y = __shfl_up_sync(0xffffffffu, incl, o);
+            if(lane >= o) {incl += y;}
+        }
+        if(threadIdx.x == 0) {sh.carry = q.slot_off;}
+        __syncthreads();
+        if(lane == 31) {sh.scan[w] = incl;}
+        if(lane == 0 && before) {atomicAdd(&sh.carry, before);}
+        __syncthreads();
+        if(w == 0)
+        {
+            const int x = sh.scan[lane];
+            int xi = x;
+#pragma unroll
+            for(int o = 1; o < 32; o <<= 1)
+            {
+                const int y = __shfl_up_sync(0xffffffffu, xi, o);
+                if(lane >= o) {xi += y;}
+            }
+            sh.scan[lane] = xi - x;
+        }
+        __syncthreads();
+        if(cell < q.ncell) {t.cell_start[q.cell_off + cell] = sh.carry + sh.scan[w] + incl - v;}
+        __syncthreads();
+    }
+    if(!bar.sync()) {return false;}
+    // participants in cell order (any order within a cell)
+    for(int e = G.thread;; e += G.nthread)
+    {
+        k = e;
+        if(!locate(mask, k, s, nslot)) {break;}
+        const int p = a.sys[s].g[g].slot_off + k;
+        t.slot_part[t.cell_start[t.part_cell[p]] + rank[p]] = p;
+    }
+    if(!bar.sync()) {return false;}
+    // each participant's slot: its rank by participant index within its cell,
+    // so that the slot order depends only on the cell assignment
+    for(int e = G.thread;; e += G.nthread)
+    {
+        k = e;
+        if(!locate(mask, k, s, nslot)) {break;}
+        const int p = a.sys[s].g[g].slot_off + k;
+        const int c = t.part_cell[p];
+        const int b = t.cell_start[c], m = t.cell_count[c];
+        const int i = t.part_particle[p];
+        const double4 x = a.pos[i];
+        int slot = b;
+        for(int u = 0; u < m; ++u) {slot += t.slot_part[b + u] < p ? 1 : 0;}
+        t.slot_particle[slot] = i;
+        t.slot_of[i]          = slot;
+        t.slot_sys[slot]      = s;
+        t.slot_pd[slot]       = make_double4(x.x, x.y, x.z, t.part_p0[p]);
+        if(t.part_p1) {t.slot_p1[slot] = t.part_p1[p];}
+    }
+    if(!bar.sync()) {return false;}
+    // narrow groups for short candidate sequences, as the launched build
+    if(t.build_lanes <= 8) {build<8>(a, g, t, mask, G, sh.narrow);}
+    else                   {build<32>(a, g, t, mask, G, sh.wide);}
+    return bar.sync();
+}
+
+// clears the flagged systems' cell counters and chunk sums for the next rebuild
+__device__ __forceinline__ void clear_cells(const Arena& a, const TermArrays& t, int g, ull mask, const Grid& G,
+                                            const Shared& sh)
+{
+    for(ull m = mask; m; m &= m - 1)
+    {
+        const int s = __ffsll((long long)m) - 1;
+        const GlobalParams& q = a.sys[s].g[g];
+        for(int c = G.thread; c < q.ncell; c += G.nthread) {t.cell_count[q.cell_off + c] = 0;}
+        const int nc = (q.ncell + CELL_CHUNK - 1) / CELL_CHUNK;
+        for(int c = G.thread; c < nc; c += G.nthread) {reinterpret_cast<int*>(t.cell_chunks)[sh.chunk_off[s][g] + c] = 0;}
+    }
+}
+
+// ------------------------------------------------------------------- forces
+
+// warp item e of term g: 32 / tpp slots, tpp lanes each (as k_pair).  The
+// slot's head, coordinates, particle and first list word are requested
+// together (every slot owns at least 32 words; those past the length are never
+// used as indices), so the chain is two loads deep: these, then the partners.
+template<int PREC, int G>
+__device__ __forceinline__ void pair_item(const Arena& a, const TermArrays& t, int e)
+{
+    const int lane = threadIdx.x & 31;
+    const int tpp = t.tpp, lt = __ffs(tpp) - 1;
+    const long long s = ((long long)e * 32 + lane) >> lt;
+    const int lg = lane & (tpp - 1);
+    const bool active = s < t.np;
+    SlotHead head{0, 0};
+    int particle = 0;
+    bool ovf = false;
+    Acc<PREC> acc;
+    if(active)
+    {
+        const long long np = t.np;
+        const bool sm = t.slot_major != 0;
+        const long long rs = sm ? tpp : np * tpp;
+        const int* nbr = t.nbr + (sm ? s * t.cap : s * tpp) + lg;
+        const double4* pd = t.slot_pd;
+        const double4 self = pd[s];
+        const int first = nbr[0];
+        particle = t.slot_particle[s];
+        head = slot_head(a, t, s);
+        const int n = head.n;
+        const PairEval<PREC, G, true, false, true, PREC == P_MIXED, true> eval(a, t, s, head.sys, self);
+        double energy = 0.0;
+        // RUN_BATCH partners requested together: words, then coordinates
+        for(int k = lg; k < n; k += RUN_BATCH * tpp)
+        {
+            int q[RUN_BATCH];
+            double4 pj[RUN_BATCH];
+            double p1[RUN_BATCH];
+#pragma unroll
+            for(int u = 0; u < RUN_BATCH; ++u)
+            {
+                q[u] = u == 0 && k == lg ? first : (k + u * tpp < n ? nbr[u * rs] : -1);
+            }
+#pragma unroll
+            for(int u = 0; u < RUN_BATCH; ++u)
+            {
+                pj[u] = q[u] >= 0 ? pd[q[u]] : self;
+                p1[u] = q[u] >= 0 ? eval.partner_p1(q[u]) : 0.0;
+            }
+            nbr += RUN_BATCH * rs;
+#pragma unroll
+            for(int u = 0; u < RUN_BATCH; ++u) {if(q[u] >= 0) {eval(pj[u], p1[u], q[u], acc, energy, ovf);}}
+        }
+    }
+    for(int o = tpp / 2; o > 0; o >>= 1) {acc.shfl_add(o);}
+    if(active && lg == 0 && head.n > 0) {add_force(a.force, particle, acc);}
+    if(ovf) {atomicOr(&a.sys[head.sys].status, ST_FIXED_OVERFLOW);}
+}
+
+template<int PREC>
+__device__ __forceinline__ void local_item(const Arena& a, const LocalArrays& l, int kind, int e)
+{
+    const long long b = (long long)e * 32 + (threadIdx.x & 31);
+    DirectAdd<PREC> W;
+    if(kind == 0)
+    {
+        if(b >= l.nbond || (a.any_frozen && a.sys[l.bond_sys[b]].frozen)) {return;}
+        if(PREC == P_FP64) {do_bond<PREC, true, false>(a, l, b, true, W);}
+        else               {do_bond_f32<PREC, true, false>(a, l, b, true, W);}
+    }
+    else if(kind == 1)
+    {
+        if(b >= l.nangle || (a.any_frozen && a.sys[l.angle_sys[b]].frozen)) {return;}
+        if(PREC == P_FP64) {do_angle<PREC, true, false>(a, l, b, true, W);}
+        else               {do_angle_f32<PREC, true, false>(a, l, b, true, W);}
+    }
+    else
+    {
+        if(b >= l.ndihd || (a.any_frozen && a.sys[l.dihd_sys[b]].frozen)) {return;}
+        if(PREC == P_FP64) {do_dihedral<PREC, true, false>(a, l, b, true, W);}
+        else               {do_dihedral_f32<PREC, true, false>(a, l, b, true, W);}
+    }
+}
+
+__host__ __device__ inline int pair_items(const TermArrays& t) {return t.on ? (int)((t.np * t.tpp + 31) / 32) : 0;}
+__host__ __device__ inline int warps_of(long long n) {return (int)((n + 31) / 32);}
+
+// The step's forces, longest items first: the dense DebyeHuckel lists, the
+// other pair terms, then the bonded terms.
+template<int PREC>
+__device__ __forceinline__ void forces(const Arena& a, const RunArgs& r, const Grid& G)
+{
+    const int n_dh = pair_items(r.t[G_DH]), n_lj = pair_items(r.t[G_LJ]), n_ex = pair_items(r.t[G_EXV]);
+    const int n_di = warps_of(r.l.ndihd), n_an = warps_of(r.l.nangle), n_bo = warps_of(r.l.nbond);
+    const int total = n_dh + n_lj + n_ex + n_di + n_an + n_bo;
+    for(int e = G.warp; e < total; e += G.nwarp)
+    {
+        int k = e;
+        if(k < n_dh) {pair_item<PREC, G_DH>(a, r.t[G_DH], k); continue;}
+        k -= n_dh;
+        if(k < n_lj) {pair_item<PREC, G_LJ>(a, r.t[G_LJ], k); continue;}
+        k -= n_lj;
+        if(k < n_ex) {pair_item<PREC, G_EXV>(a, r.t[G_EXV], k); continue;}
+        k -= n_ex;
+        if(k < n_di) {local_item<PREC>(a, r.l, 2, k); continue;}
+        k -= n_di;
+        if(k < n_an) {local_item<PREC>(a, r.l, 1, k); continue;}
+        local_item<PREC>(a, r.l, 0, k - n_an);
+    }
+}
+
+// --------------------------------------------------------------------- steps
+
+template<int PREC, bool AUX>
+__global__ void __launch_bounds__(RT, 1) k_run(const __grid_constant__ RunArgs r)
+{
+    __shared__ Shared sh;
+    extern __shared__ __align__(16) unsigned char dyn[];
+    SysDev* const sys = reinterpret_cast<SysDev*>(dyn);
+    Arena a = r.a;
+    a.sys = sys;
+    const int nsys = a.nsys;
+    const Grid G;
+    Barrier bar{r.barrier, &r.a.sys[0].status, r.cluster != 0, 0u};
+    const unsigned full = 0xffffffffu;
+    {
+        static_assert(sizeof(SysDev) % sizeof(int4) == 0, "copied in 16-byte words");
+        const int4* src = reinterpret_cast<const int4*>(r.a.sys);
+        for(int w = threadIdx.x; w < nsys * (int)(sizeof(SysDev) / sizeof(int4)); w += RT) {reinterpret_cast<int4*>(dyn)[w] = src[w];}
+        for(int w = threadIdx.x; w < nsys * NGLOBAL; w += RT) {(&sh.rebuilds[0][0])[w] = 0;}
+    }
+    __syncthreads();
+    if(threadIdx.x < NGLOBAL)
+    {
+        int c = 0;
+        for(int s = 0; s < nsys; ++s)
+        {
+            sh.chunk_off[s][threadIdx.x] = c;
+            c += (sys[s].g[threadIdx.x].ncell + CELL_CHUNK - 1) / CELL_CHUNK;
+        }
+    }
+    __syncthreads();
+    for(int g = 0; g < NGLOBAL; ++g)
+    {
+        if(!r.t[g].on) {continue;}
+        for(int c = G.thread; c < r.t[g].ncell; c += G.nthread) {r.t[g].cell_count[c] = 0;}
+        const int nc = sh.chunk_off[nsys - 1][g] + (sys[nsys - 1].g[g].ncell + CELL_CHUNK - 1) / CELL_CHUNK;
+        for(int c = G.thread; c < nc; c += G.nthread) {reinterpret_cast<int*>(r.t[g].cell_chunks)[c] = 0;}
+    }
+    ull* const disp = r.disp2;                    // [2][nsys], zero between launches
+
+    // this thread's first particle and its noise, drawn while the grid waits
+    const long long i0 = G.thread;
+    const int sys0 = i0 < a.n ? a.psys[i0] : -1;
+    const int kind0 = sys0 >= 0 ? sys[sys0].integrator : I_VV;
+    const bool noisy0 = sys0 >= 0 && !sys[sys0].frozen && (kind0 == I_BAOAB || kind0 == I_GBAOAB || (AUX && kind0 == I_GJF));
+    double n0 = 0.0, n1 = 0.0, n2 = 0.0;
+    auto draw = [&](int k) {
+        if(noisy0) {const SysDev& S = sys[sys0]; gaussian3(S.seed, (ull)(i0 - S.off), S.step + k, n0, n1, n2);}
+    };
+    draw(0);
+
+    for(int k = 0; k < r.nsteps; ++k)
+    {
+        ull* const d = disp + (k & 1) * nsys;
+        // ---- integrator pass
+        for(long long i = i0; i - (threadIdx.x & 31) < a.n; i += G.nthread)
+        {
+            const int s = i == i0 ? sys0 : (i < a.n ? a.psys[i] : -1);
+            double d2 = 0.0;
+            if(s >= 0 && !sys[s].frozen)
+            {
+                SysDev& S = sys[s];
+                const ull step = S.step + k;
+                d2 = advance_particle<PREC, AUX>(a, S, i, k > 0 || r.kick, step, [&](double& x, double& y, double& z) {
+                    if(i == i0) {x = n0; y = n1; z = n2;}
+                    else        {gaussian3(S.seed, (ull)(i - S.off), step, x, y, z);}
+                });
+            }
+            const int s0 = __shfl_sync(full, s, 0);
+            if(__all_sync(full, s == s0 || s < 0))
+            {
+                double m = d2;
+#pragma unroll
+                for(int o = 16; o > 0; o >>= 1) {m = fmax(m, __shfl_xor_sync(full, m, o));}
+                if((threadIdx.x & 31) == 0) {atomicMax(&d[s0], (ull)__double_as_longlong(m));}
+            }
+            else if(s >= 0) {atomicMax(&d[s], (ull)__double_as_longlong(d2));}
+        }
+        if(threadIdx.x < NGLOBAL) {sh.flag[threadIdx.x] = 0;}
+        if(!bar.sync()) {return;}
+        // ---- reduce_margin of every system (core/PeriodicGridCellList.hpp:100-110),
+        // by every block for itself
+        for(int s = threadIdx.x; s < nsys; s += RT)
+        {
+            SysDev& S = sys[s];
+            if(S.frozen) {continue;}
+            const double dd = 2 * sqrt(__longlong_as_double((long long)d[s]));
+            for(int g = 0; g < NGLOBAL; ++g)
+            {
+                GlobalParams& P = S.g[g];
+                if(!r.t[g].on || !P.on) {continue;}
+                P.current_margin = __dsub_rn(P.current_margin, dd);
+                if(P.current_margin < 0)
+                {
+                    atomicOr(&sh.flag[g], 1ull << s);
+                    P.current_margin = __dmul_rn(P.cutoff, P.margin);
+                    sh.rebuilds[s][g] += 1;
+                }
+            }
+        }
+        // the other displacement buffer, read by every block before the last barrier
+        if(blockIdx.x == 0) {for(int s = threadIdx.x; s < nsys; s += RT) {disp[((k & 1) ^ 1) * nsys + s] = 0;}}
+        __syncthreads();
+        if(sh.flag[G_EXV] && !rebuild<G_EXV>(a, r.t[G_EXV], sh.flag[G_EXV], G, sh, bar)) {return;}
+        if(sh.flag[G_DH] && !rebuild<G_DH>(a, r.t[G_DH], sh.flag[G_DH], G, sh, bar)) {return;}
+        if(sh.flag[G_LJ] && !rebuild<G_LJ>(a, r.t[G_LJ], sh.flag[G_LJ], G, sh, bar)) {return;}
+        // ---- forces
+        forces<PREC>(a, r, G);
+        for(int g = 0; g < NGLOBAL; ++g) {if(sh.flag[g]) {clear_cells(a, r.t[g], g, sh.flag[g], G, sh);}}
+        bar.arrive();
+        draw(k + 1);                              // while the others finish
+        if(!bar.wait()) {return;}
+    }
+    // ---- closing half of the last step, counters
+    if(r.close)
+    {
+        for(long long i = i0; i < a.n; i += G.nthread)
+        {
+            const int s = a.psys[i];
+            if(!sys[s].frozen) {close_particle<PREC>(a, sys[s], i, sys[s].step + r.nsteps);}
+        }
+    }
+    __syncthreads();
+    for(int s = threadIdx.x; s < nsys; s += RT)
+    {
+        SysDev& S = r.a.sys[s];
+        if(sys[s].status) {atomicOr(&S.status, sys[s].status);}
+        if(blockIdx.x != 0) {continue;}
+        disp[s] = 0;
+        disp[nsys + s] = 0;
+        if(sys[s].frozen) {continue;}
+        S.step = sys[s].step + r.nsteps;
+        for(int g = 0; g < NGLOBAL; ++g)
+        {
+            S.g[g].current_margin = sys[s].g[g].current_margin;
+            S.g[g].rebuilds += sh.rebuilds[s][g];
+        }
+    }
+}
+
+}  // namespace
+
+cudaError_t launch_run(RunArgs r, int sms, cudaStream_t s)
+{
+    // blocks: a warp per item of the force phase, at most one block per SM
+    int items = 0;
+    for(int g = 0; g < NGLOBAL; ++g) {items += pair_items(r.t[g]);}
+    items += warps_of(r.l.nbond) + warps_of(r.l.nangle) + warps_of(r.l.ndihd);
+    items = std::max(items, warps_of(r.a.n));
+    int blocks = std::max(1, std::min(sms, (items + RT / 32 - 1) / (RT / 32)));
+    r.cluster = blocks <= RUN_CLUSTER_MAX ? 1 : 0;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(blocks);
+    cfg.blockDim = dim3(RT);
+    cfg.stream = s;
+    cudaLaunchAttribute at{};
+    if(r.cluster)
+    {
+        at.id = cudaLaunchAttributeClusterDimension;
+        at.val.clusterDim.x = blocks;
+        at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    }
+    else
+    {
+        at.id = cudaLaunchAttributeCooperative;
+        at.val.cooperative = 1;
+    }
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    cfg.dynamicSmemBytes = sizeof(SysDev) * r.a.nsys;
+    const bool aux = r.a.accel != nullptr;
+    auto* kernel = r.a.precision == P_FP64 ? (aux ? k_run<P_FP64, true> : k_run<P_FP64, false>)
+                                           : (aux ? k_run<P_MIXED, true> : k_run<P_MIXED, false>);
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               (int)(sizeof(SysDev) * RUN_MAX_SYSTEMS));
+    if(e != cudaSuccess) {return e;}
+    note_launches(1);
+    return cudaLaunchKernelEx(&cfg, kernel, r);
+}
+
+}  // namespace mjg

@@ -1,0 +1,91 @@
+"""The multi-step kernel of small arenas against the step's own launches
+(graphs off): the same bits in the mixed form, the order of the FP64 sums apart
+in the plain form.  Sizes at the edges of its split: less than a warp, one
+cluster, a ragged last warp, several particles per thread, several systems."""
+import numpy as np
+import pytest
+
+from mjolnir_b200 import systems as S
+from mjolnir_b200.engine import Engine
+
+pytestmark = pytest.mark.gpu
+
+
+def cube(d):
+    r = float(np.abs(d.pos).max()) + 2.0
+    d.boundary, d.lower, d.upper = "PeriodicCuboid", (-r, -r, -r), (r, r, r)
+    return d
+
+
+def systems(name):
+    if name == "beads_5":                       # no list has a partner for long
+        return [S.polymer_melt(nchains=1, nbeads=5, radius=30.0, seed=3, charged_fraction=0.9)]
+    if name == "chain_33":
+        return [S.polymer_melt(nchains=1, nbeads=33, radius=40.0, seed=4, margin=0.1)]
+    if name == "melt_cube":
+        return [cube(S.polymer_melt(nchains=9, nbeads=111, radius=55.0, seed=5, margin=0.15))]
+    if name == "lj":
+        return [S.lj_fluid(n=4096, margin=0.1, seed=6)]
+    if name == "fluid_40001":                   # several pair items per warp, cells of many members
+        return [S.bead_fluid(n=40001, density=0.003, seed=7, margin=0.1, dt=0.6)]
+    out = [S.polymer_melt(nchains=4, nbeads=50, radius=50.0, seed=31, margin=0.1), S.lj_fluid(n=343, seed=32, margin=0.05),
+           S.bead_fluid(n=1500, density=0.003, seed=33, dt=0.6, margin=0.1),
+           cube(S.polymer_melt(nchains=3, nbeads=41, radius=40.0, seed=34, margin=0.1))]
+    if name == "integrators":
+        for d, kind in zip(out, ("UnderdampedLangevin", "VelocityVerlet", "G-JFLangevin", "g-BAOABLangevin")):
+            d.integrator = kind
+        return out
+    return [d for k in range(16) for d in (S.polymer_melt(nchains=1, nbeads=20 + 7 * k, radius=40.0, seed=50 + k, margin=0.1),
+                                           out[k % 4])]     # 32 systems
+
+
+def run(name, precision, graphs, half=False, frozen=False, steps=(1, 37, 62)):
+    descs = systems(name)
+    e = Engine(precision, graphs=graphs)
+    ids = [e.add_system(d) for d in descs]
+    if half:
+        for t in ("exv", "dh", "lj"):
+            e.set_half_lists(t, True)
+    e.commit()
+    if frozen:
+        e.freeze(ids[1])
+    n0 = e.launch_count()
+    for k in steps:
+        e.step(k)
+    launches = e.launch_count() - n0
+    out = []
+    for sid, d in zip(ids, descs):
+        terms = [t for t in ("exv", "dh", "lj") if getattr(d, t) is not None]
+        out.append((e.state(sid), e.step_count(sid), [e.rebuild_count(sid, t) for t in terms],
+                    [e.neighbors(sid, t) for t in terms]))
+    e.close()
+    return out, launches
+
+
+@pytest.mark.parametrize("name", ["beads_5", "chain_33", "melt_cube", "lj", "fluid_40001", "integrators", "many"])
+@pytest.mark.parametrize("precision", ["mixed", "fp64"])
+def test_steps_of_one_launch_equal_the_launched_steps(name, precision):
+    got, few = run(name, precision, True)
+    want, many = run(name, precision, False)
+    assert few < many / 20
+    for g, w in zip(got, want):
+        assert g[1] == w[1] and g[2] == w[2]
+        assert all(np.array_equal(x, y) for x, y in zip(g[3], w[3]))
+        for x, y in zip(g[0], w[0]):
+            if precision == "mixed":
+                assert np.array_equal(x, y)
+            else:
+                # the sums of a step differ by rounding (1e-16 of the terms); 100 steps of these systems
+                # amplify that by less than a factor of 1e4 (the liquid's e-fold is about 40 steps)
+                assert np.abs(x - y).max() <= 1e-10 * max(1.0, np.abs(y).max())
+    assert any(any(c > 0 for c in g[2]) for g in got) or name == "beads_5"
+
+
+@pytest.mark.parametrize("half,frozen", [(True, False), (False, True), (True, True)])
+def test_half_lists_and_frozen_systems(half, frozen):
+    got, _ = run("many", "mixed", True, half, frozen)
+    want, _ = run("many", "mixed", False, False, frozen)
+    for g, w in zip(got, want):
+        assert g[1] == w[1] and g[2] == w[2]
+        for x, y in zip(g[0], w[0]):
+            assert np.array_equal(x, y)
