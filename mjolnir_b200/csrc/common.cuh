@@ -104,6 +104,16 @@ __device__ __forceinline__ long long fx_from_double(double v)
     const double s = v * FX_SCALE + FX_MAGIC;
     return __double_as_longlong(s) - __double_as_longlong(FX_MAGIC);
 }
+// The mixed form's plain pair force, an FP32 coefficient c times an FP64
+// displacement d, on the grid: c is scaled in FP32 (exactly, by a power of two;
+// a product that leaves FP32 there is far outside the range that the caller
+// checks) and one fused product-sum rounds c d 2^FX_SHIFT to an integer.  Odd in
+// d and in c, as round to nearest even is.
+__device__ __forceinline__ double fx_coefficient(float c) {return (double)(c * (float)FX_SCALE);}
+__device__ __forceinline__ long long fx_product(double scaled_c, double d)
+{
+    return __double_as_longlong(fma(scaled_c, d, FX_MAGIC)) - __double_as_longlong(FX_MAGIC);
+}
 __device__ __forceinline__ double fx_to_double(long long v)
 {
     return (double)v * FX_INV_SCALE;

@@ -85,7 +85,7 @@ struct Window {
 __device__ __forceinline__ double3 direction(const SysDev& S, const double4& from, const double4& to)
 {
     double3 d = make_double3(to.x - from.x, to.y - from.y, to.z - from.z);
-    if(S.boundary == B_PERIODIC)
+    if(image_needed(d.x, d.y, d.z, S.halfw_hi))
     {
         d.x = min_image(d.x, S.halfw[0], S.width[0]);
         d.y = min_image(d.y, S.halfw[1], S.width[1]);

@@ -7,6 +7,41 @@
 
 namespace mjg {
 
+// Single-instruction forms of the mixed form's reciprocal root and power of
+// two.  Squared distances and exponents of listed pairs are normal numbers, for
+// which these round as the general forms do, which spend as many instructions
+// again on subnormal ones; a subnormal squared distance gives an infinite force
+// either way, which the fixed-point range check reports.
+__device__ __forceinline__ float rsqrt_approx(float x)
+{
+    float y;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+__device__ __forceinline__ float exp2_approx(float x)
+{
+    float y;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+// 1 / x: the hardware's approximation and one Newton step, r + r (1 - x r),
+// which leaves the rounding of the last product-sum (at most 1 ulp, and the
+// nearest float in nearly all cases).
+__device__ __forceinline__ float reciprocal(float x)
+{
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return fmaf(r, fmaf(-x, r, 1.0f), r);
+}
+
+// slot coordinates and parameter in one 32-byte load (32-byte aligned)
+__device__ __forceinline__ double4 load_pd(const double4* p)
+{
+    double4 v;
+    asm volatile("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(v.x), "=d"(v.y), "=d"(v.z), "=d"(v.w) : "l"(p));
+    return v;
+}
+
 template<int PREC>
 struct Acc;
 
@@ -43,17 +78,16 @@ template<> struct Acc<P_MIXED>
         x += fx_from_double(fx); y += fx_from_double(fy); z += fx_from_double(fz);
     }
     // the mixed form's plain potentials: the FP32 pair coefficient c times
-    // the FP64 displacement, each component rounded to the fixed-point grid
-    // on the FP64 pipe (one conversion per pair instead of one per component
-    // and coordinate); `bound` >= |c| |r| (|c| max(|r|^2, 1) or |c| |r|, in
+    // the FP64 displacement, each component rounded once to the fixed-point
+    // grid (fx_product); `bound` >= |c| |r| (|c| max(|r|^2, 1) or |c| |r|, in
     // FP32) flags a force outside the fixed-point range
     __device__ __forceinline__ void add_c(float c, float bound, double dx, double dy, double dz, bool& ovf)
     {
-        const double cd = (double)c;
+        const double cs = fx_coefficient(c);
         ovf |= !(bound < (float)(FX_LIMIT * FX_INV_SCALE));
-        x += fx_from_double(cd * dx);
-        y += fx_from_double(cd * dy);
-        z += fx_from_double(cd * dz);
+        x += fx_product(cs, dx);
+        y += fx_product(cs, dy);
+        z += fx_product(cs, dz);
     }
     __device__ __forceinline__ void shfl_add(int o)
     {
@@ -83,8 +117,8 @@ struct PairEval {
     double4 pi;
     long long s;
     int halfw_hi;               // image_needed
-    double crsq, coefc, eps, eps12, debye, inv_debye, abs_cut_sq, qi, inv4pi, epsi, cr;
-    float eps12f, epsf, coefcf, debf, invdf, crsqf, wif;
+    double crsq, coefc, eps, eps12, inv_debye, abs_cut_sq, qi, inv4pi, epsi, cr;
+    float eps12f, epsf, coefcf, invdf, crsqf, wif;
     int kind, power;
     bool half;                  // HALF_RT: half lists
     bool fe;                    // energy-only: the force-and-energy rule of the generic loop
@@ -109,14 +143,14 @@ struct PairEval {
         coefc = P.coef_at_cutoff;
         eps   = P.eps;
         eps12 = eps * 12;
-        debye = P.debye; inv_debye = P.inv_debye;
+        inv_debye = P.inv_debye;
         abs_cut_sq = P.abs_cutoff * P.abs_cutoff;
         qi = pi.w; inv4pi = P.inv4pi;
         slot_p1 = t.slot_p1;
         // second per-slot parameter: LJ-family epsilon, HardCore core radius
         epsi  = (G == G_LJ || (G == G_EXV && kind == EXV_HARD_CORE)) ? t.slot_p1[slot] : 0.0;
         eps12f = (float)eps12; epsf = (float)eps; coefcf = (float)coefc;
-        debf = (float)debye; invdf = (float)inv_debye;
+        invdf = (float)inv_debye;
         crsqf = (float)crsq; wif = (float)pi.w;
         half = !HALF_RT || t.half != 0;
         fe = !NF && t.fe_energy != 0;
@@ -124,13 +158,9 @@ struct PairEval {
         slot_particle = t.slot_particle;
     }
 
-    // The second parameter of partner q, for the potentials that have one:
+    // The Lennard-Jones family's second parameter of partner q (epsilon):
     // callers request it with the partner's coordinates.
-    __device__ __forceinline__ double partner_p1(int q) const
-    {
-        if(G == G_LJ || (G == G_EXV && kind == EXV_HARD_CORE)) {return slot_p1[q];}
-        return 0.0;
-    }
+    __device__ __forceinline__ double partner_p1(int q) const {return G == G_LJ ? slot_p1[q] : 0.0;}
 
     // Half lists (mixed form): the partner's share of the pair, the negated
     // fixed-point components of c r_ij.  Its own evaluation of the pair would
@@ -146,6 +176,22 @@ struct PairEval {
         {
             if((HALF_RT && !half) || c == 0.0) {return;}
             const long long x = fx_from_double(c * dx), y = fx_from_double(c * dy), z = fx_from_double(c * dz);
+            unsigned long long* f =
+                reinterpret_cast<unsigned long long*>(static_cast<longlong4*>(force) + (jp >= 0 ? jp : slot_particle[q]));
+            if(x) {atomicAdd(f + 0, (unsigned long long)(-x));}
+            if(y) {atomicAdd(f + 1, (unsigned long long)(-y));}
+            if(z) {atomicAdd(f + 2, (unsigned long long)(-z));}
+        }
+    }
+
+    // The same for an FP32 coefficient (Acc::add_c).
+    __device__ __forceinline__ void partner_add_c(float c, int q, double dx, double dy, double dz, int jp) const
+    {
+        if constexpr(PREC == P_MIXED && NF && HALF)
+        {
+            if((HALF_RT && !half) || c == 0.0f) {return;}
+            const double cs = fx_coefficient(c);
+            const long long x = fx_product(cs, dx), y = fx_product(cs, dy), z = fx_product(cs, dz);
             unsigned long long* f =
                 reinterpret_cast<unsigned long long*>(static_cast<longlong4*>(force) + (jp >= 0 ? jp : slot_particle[q]));
             if(x) {atomicAdd(f + 0, (unsigned long long)(-x));}
@@ -314,7 +360,7 @@ struct PairEval {
         {
             if(kind != EXV_PLAIN)
             {
-                const double radius = kind == EXV_HARD_CORE ? epsi + p1j : 0.0;
+                const double radius = kind == EXV_HARD_CORE ? epsi + slot_p1[q] : 0.0;
                 exv_family(pi.w + pj.w, radius, l2, dx, dy, dz, count_e, acc, energy, ovf, q, jp);
                 return;
             }
@@ -335,7 +381,7 @@ struct PairEval {
                 // branch-free: every lane evaluates, pairs outside the
                 // cutoff add an exact zero; sigma in FP32 from the two radii
                 const float l2f = (float)l2;
-                const float rcp = __frcp_rn(l2f);
+                const float rcp = reciprocal(l2f);
                 const float sg = wif + (float)pj.w;
                 const float s2 = sg * sg * rcp;
                 const float s6 = s2 * s2 * s2;
@@ -343,7 +389,7 @@ struct PairEval {
                 if constexpr(NF)
                 {
                     acc.add_c(cf, fabsf(cf) * fmaxf(l2f, 1.0f), dx, dy, dz, ovf);
-                    partner_add((double)cf, q, dx, dy, dz, jp);
+                    partner_add_c(cf, q, dx, dy, dz, jp);
                 }
                 if(count_e && in) {energy += (double)(epsf * (s6 * s6 - coefcf));}
             }
@@ -358,26 +404,27 @@ struct PairEval {
                 const double rl = rsqrt(l2);
                 const double l  = l2 * rl;
                 const double ex = exp(-l * inv_debye);
-                if(NF) {acc.add(-qq * (debye + l) * inv_debye / (l * l) * ex * rl, dx, dy, dz, ovf);}
+                if(NF) {acc.add(-qq * fma(l, inv_debye, 1.0) * (rl * rl) * ex * rl, dx, dy, dz, ovf);}
                 if(count_e) {energy += qq * (ex / l - coefc);}
             }
             else
             {
                 // branch-free like ExcludedVolume: outside the cutoff the
-                // distance is replaced by the cutoff and the force is zero
+                // force is zero; (debye + l) / debye = 1 + l / debye;
                 // the charge product stays in FP64 and scales the FP32
                 // coefficient of the unit-charge potential
                 const double qq = (qi * pj.w) * inv4pi;
-                const float l2f = in ? (float)l2 : (float)abs_cut_sq;
-                const float rl = rsqrtf(l2f);
+                const float l2f = (float)l2;
+                const float rl = rsqrt_approx(l2f);
                 const float l  = l2f * rl;
-                const float ex = __expf(-l * invdf);
-                const float cu = in ? -(debf + l) * invdf * (rl * rl) * ex * rl : 0.0f;
+                const float ex = exp2_approx(__fmul_rn(l, invdf) * -1.4426950408889634f);
+                // an explicit product-sum: every kernel must round alike
+                const float cu = in ? -fmaf(l, invdf, 1.0f) * (rl * rl) * rl * ex : 0.0f;
                 if constexpr(NF)
                 {
                     const float cf = (float)qq * cu;
                     acc.add_c(cf, fabsf(cf) * l, dx, dy, dz, ovf);
-                    partner_add((double)cf, q, dx, dy, dz, jp);
+                    partner_add_c(cf, q, dx, dy, dz, jp);
                 }
                 if(count_e && in) {energy += qq * (double)(ex * rl - coefcf);}
             }
@@ -405,15 +452,15 @@ struct PairEval {
             else
             {
                 const float l2f = (float)l2;
-                const float rcp = __frcp_rn(l2f);
+                const float rcp = reciprocal(l2f);
                 const float s2 = (float)sigma_sq * rcp;
                 const float s6 = s2 * s2 * s2;
                 const float ef = (float)epsilon;
                 if constexpr(NF)
                 {
-                    const float cf = 24.0f * ef * (s6 - 2.0f * s6 * s6) * rcp;
+                    const float cf = 24.0f * ef * fmaf(-2.0f * s6, s6, s6) * rcp;
                     acc.add_c(cf, fabsf(cf) * fmaxf(l2f, 1.0f), dx, dy, dz, ovf);
-                    partner_add((double)cf, q, dx, dy, dz, jp);
+                    partner_add_c(cf, q, dx, dy, dz, jp);
                 }
                 if(count_e) {energy += (double)(4.0f * ef * (s6 * s6 - s6 - coefcf));}
             }

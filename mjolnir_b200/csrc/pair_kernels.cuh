@@ -104,47 +104,54 @@ __global__ void __launch_bounds__(TPB, 4) k_pair(Arena a, TermArrays t)
         s = first + sorted_group<TPB / TPP>(a, t, first, (int)(threadIdx.x / TPP), lg == 0, TPP * UNR, head);
     }
     const bool active = s < t.np;
-    if(!SORT && active) {head = slot_head(a, t, s);}
-    const int sys = head.sys;
     double energy = 0.0;
     bool ovf = false;
     Acc<PREC> acc;
-    if(active && head.n > 0)         // the group's slot; an empty list reads nothing
+    int particle = 0;
+    if(active && (!SORT || head.n > 0))    // a sorted group knows that its list is empty
     {
-        const PairEval<PREC, G, NF, NE, PER, HALF> eval(a, t, s, sys);
-        const long long np = t.np;
-        const int n = head.n;
         // word k = lg + r TPP of the slot's list: blocked layout, rows np TPP
         // words apart; slot-major layout, the slot's cap words in a row, the
         // whole list requested into L2 (16-byte aligned: cap is a multiple of
         // 32 words) before the walk starts
         const bool sm = t.slot_major != 0;
-        const long long rs = sm ? TPP : np * TPP;
+        const long long rs = sm ? TPP : t.np * TPP;
         const int* __restrict__ nbr = t.nbr + (sm ? s * t.cap : s * TPP) + lg;
-        if(sm && lg == 0 && n > 0) {bulk_prefetch_l2(t.nbr + s * t.cap, (unsigned)((n + 3) / 4) * 16u);}
         const double4* __restrict__ pd = t.slot_pd;
+        // the slot's coordinates, particle and first list word are requested
+        // with its head (every slot owns cap >= TPP words; a word past the
+        // length is never used as an index), so the walk starts one load
+        // latency after the launch
+        const double4 self = load_pd(pd + s);
+        int q = __ldg(nbr);
+        particle = t.slot_particle[s];
+        if(!SORT) {head = slot_head(a, t, s);}
+        const int n = head.n;
+        if(sm && lg == 0 && n > 0) {bulk_prefetch_l2(t.nbr + s * t.cap, (unsigned)((n + 3) / 4) * 16u);}
+        if(n > 0)
+        {
+        const PairEval<PREC, G, NF, NE, PER, HALF> eval(a, t, s, head.sys, self);
         if(UNR == 1)
         {
             // software pipeline: the next partner's index and coordinates are
             // requested before the current pair is evaluated
-            // the first list word is read whatever the list's length (every
-            // slot owns cap >= TPP words), so that its load does not wait for
-            // the length; a word past the length is never used as an index
             int k = lg;
-            int q = __ldg(nbr);
-            double4 pj = make_double4(0.0, 0.0, 0.0, 0.0);
-            if(k < n) {pj = pd[q];}
+            double4 pj = self;
+            double p1 = 0.0;
+            if(k < n) {pj = load_pd(pd + q); p1 = eval.partner_p1(q);}
             for(; k < n; k += TPP)
             {
                 const int kn = k + TPP;
-                const int kp = k + PF_ROWS * TPP;
-                if(!sm && kp < n) {prefetch_l2(nbr + (long long)(kp / TPP) * rs);}
+                nbr += rs;
+                if(!sm && k + PF_ROWS * TPP < n) {prefetch_l2(nbr + (PF_ROWS - 1) * rs);}
                 int qn = q;
                 double4 pn = pj;
-                if(kn < n) {qn = __ldg(nbr + (long long)(kn / TPP) * rs); pn = pd[qn];}
-                eval(pj, eval.partner_p1(q), q, acc, energy, ovf);
+                double p1n = p1;
+                if(kn < n) {qn = __ldg(nbr); pn = load_pd(pd + qn); p1n = eval.partner_p1(qn);}
+                eval(pj, p1, q, acc, energy, ovf);
                 q = qn;
                 pj = pn;
+                p1 = p1n;
             }
         }
         else
@@ -153,32 +160,37 @@ __global__ void __launch_bounds__(TPB, 4) k_pair(Arena a, TermArrays t)
             {
                 int qv[UNR];
                 double4 pv[UNR];
+                double p1v[UNR];
 #pragma unroll
                 for(int u = 0; u < UNR; ++u)
                 {
                     const int kp = k + (PF_ROWS + u) * TPP;
-                    if(!sm && kp < n) {prefetch_l2(nbr + (long long)(kp / TPP) * rs);}
+                    if(!sm && kp < n) {prefetch_l2(nbr + (PF_ROWS + u) * rs);}
                 }
 #pragma unroll
                 for(int u = 0; u < UNR; ++u)
                 {
                     const int kk = k + u * TPP;
-                    qv[u] = kk < n ? __ldg(nbr + (long long)(kk / TPP) * rs) : -1;
+                    qv[u] = kk < n ? (u == 0 && k == lg ? q : __ldg(nbr + u * rs)) : -1;
                 }
-#pragma unroll
-                for(int u = 0; u < UNR; ++u) {pv[u] = qv[u] >= 0 ? pd[qv[u]] : eval.pi;}
 #pragma unroll
                 for(int u = 0; u < UNR; ++u)
                 {
-                    if(qv[u] >= 0) {eval(pv[u], eval.partner_p1(qv[u]), qv[u], acc, energy, ovf);}
+                    pv[u] = qv[u] >= 0 ? load_pd(pd + qv[u]) : self;
+                    p1v[u] = qv[u] >= 0 ? eval.partner_p1(qv[u]) : 0.0;
                 }
+#pragma unroll
+                for(int u = 0; u < UNR; ++u) {if(qv[u] >= 0) {eval(pv[u], p1v[u], qv[u], acc, energy, ovf);}}
+                nbr += UNR * rs;
             }
         }
+        }
     }
+    const int sys = head.sys;
     // group reduction: exact in fixed point, fixed order in FP64
 #pragma unroll
     for(int o = TPP / 2; o > 0; o >>= 1) {acc.shfl_add(o);}
-    if(active && NF && lg == 0) {acc.store(a.force, t.slot_particle[s]);}
+    if(NF && lg == 0 && head.n > 0) {acc.store(a.force, particle);}
     if(ovf) {atomicOr(&a.sys[sys].status, ST_FIXED_OVERFLOW);}
     if(NE)
     {
@@ -239,23 +251,28 @@ __global__ void __launch_bounds__(TPB, 4) k_pair_vec(Arena a, TermArrays t)
         const long long first = (long long)blockIdx.x * TPB;
         s = first + sorted_group<TPB>(a, t, first, (int)threadIdx.x, true, L, head);
     }
-    if(s >= t.np) {return;}
-    if(!SORT) {head = slot_head(a, t, s);}
-    if(head.n == 0) {return;}        // an empty list (frequent in half lists): nothing to add
+    if(s >= t.np || (SORT && head.n == 0)) {return;}   // an empty list (frequent in half lists): nothing to add
+    // the slot's coordinates, particle and first block of words are requested
+    // with its head (every slot owns cap >= L words; words past the length are
+    // never used as indices)
+    const double4 self = load_pd(t.slot_pd + s);
+    int q[L];
+    load_block<L>(t.nbr + s * L, q);
+    const int particle = t.slot_particle[s];
+    if(!SORT)
+    {
+        head = slot_head(a, t, s);
+        if(head.n == 0) {return;}
+    }
     const int sys = head.sys;
     double energy = 0.0;
     bool ovf = false;
     Acc<PREC> acc;
-    const PairEval<PREC, G, true, false, PER, HALF> eval(a, t, s, sys);
+    const PairEval<PREC, G, true, false, PER, HALF> eval(a, t, s, sys, self);
     const long long np = t.np;
     const int n = head.n;
     const double4* __restrict__ pd = t.slot_pd;
     constexpr int W = L < 4 ? L : 4;                 // partners requested together
-    // the first block is read whatever the list's length (every slot owns
-    // cap >= L words), so that its load does not wait for the length; words
-    // past the length are never used as indices
-    int q[L];
-    load_block<L>(t.nbr + s * L, q);
     for(int k = 0; k < n; k += L)
     {
         int qn[L];
@@ -270,7 +287,7 @@ __global__ void __launch_bounds__(TPB, 4) k_pair_vec(Arena a, TermArrays t)
 #pragma unroll                                       // their coordinates, so the atomics wait on nothing
             for(int u = 0; u < W; ++u)
             {
-                pv[u] = u0 + u < m ? pd[q[u0 + u]] : eval.pi;
+                pv[u] = u0 + u < m ? load_pd(pd + q[u0 + u]) : self;
                 jv[u] = HALF && u0 + u < m ? t.slot_particle[q[u0 + u]] : -1;
             }
 #pragma unroll
@@ -279,7 +296,7 @@ __global__ void __launch_bounds__(TPB, 4) k_pair_vec(Arena a, TermArrays t)
 #pragma unroll
         for(int u = 0; u < L; ++u) {q[u] = qn[u];}
     }
-    acc.store(a.force, t.slot_particle[s]);
+    acc.store(a.force, particle);
     if(ovf) {atomicOr(&a.sys[sys].status, ST_FIXED_OVERFLOW);}
 }
 
@@ -351,7 +368,7 @@ __global__ void __launch_bounds__(TPB) k_pair_warp(Arena a, TermArrays t)
                 qv[u] = kk < kend ? __ldg(nbr + (((long long)(kk >> lt) * np + s) << lt) + (kk & (tpp - 1))) : -1;
             }
 #pragma unroll
-            for(int u = 0; u < UNR; ++u) {pv[u] = qv[u] >= 0 ? pd[qv[u]] : eval.pi;}
+            for(int u = 0; u < UNR; ++u) {pv[u] = qv[u] >= 0 ? load_pd(pd + qv[u]) : eval.pi;}
 #pragma unroll
             for(int u = 0; u < UNR; ++u)
             {

@@ -323,7 +323,7 @@ __device__ __forceinline__ void pair_item(const Arena& a, const TermArrays& t, i
         const long long rs = sm ? tpp : np * tpp;
         const int* nbr = t.nbr + (sm ? s * t.cap : s * tpp) + lg;
         const double4* pd = t.slot_pd;
-        const double4 self = pd[s];
+        const double4 self = load_pd(pd + s);
         const int first = nbr[0];
         particle = t.slot_particle[s];
         head = slot_head(a, t, s);
@@ -344,7 +344,7 @@ __device__ __forceinline__ void pair_item(const Arena& a, const TermArrays& t, i
 #pragma unroll
             for(int u = 0; u < RUN_BATCH; ++u)
             {
-                pj[u] = q[u] >= 0 ? pd[q[u]] : self;
+                pj[u] = q[u] >= 0 ? load_pd(pd + q[u]) : self;
                 p1[u] = q[u] >= 0 ? eval.partner_p1(q[u]) : 0.0;
             }
             nbr += RUN_BATCH * rs;
