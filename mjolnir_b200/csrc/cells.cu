@@ -3,22 +3,28 @@
 // Replaces PeriodicGridCellList::make / UnlimitedGridCellList::make
 // (core/PeriodicGridCellList.hpp:198-351, core/UnlimitedGridCellList.hpp
 // :152-255) for every system of the arena that reduce_margin flagged.  A
-// planning kernel turns the flagged systems into a work list of 256-item
-// chunks (participants and cells); every later kernel is a persistent grid
-// that walks only those chunks, so a step in which 5 of 256 systems rebuild
-// costs 5 systems' worth of work:
-//   1. zero the flagged systems' cell counters,
-//   2. bin their participants (one atomic increment per participant),
-//   3. exclusive scan of each flagged system's cells (one block per system),
-//   4. scatter participants into cell order, sort each cell by participant,
-//   5. renumber: slot = position in cell order (spatially coherent slots),
-//   6. build each slot's partner list from the 27 neighbouring cells (one
-//      warp per slot) with the reference's membership test, evaluated in FP64
-//      without contraction:
+// planning kernel turns the flagged systems into a work list of chunks
+// (participants and cells); every later kernel is a persistent grid that walks
+// only those chunks, so a step in which 5 of 256 systems rebuild costs 5
+// systems' worth of work:
+//   1. bin the flagged systems' participants (one atomic increment per
+//      participant, which gives its place within its cell),
+//   2. exclusive scan of the cells, chunk by chunk (each chunk adds up the sums
+//      of its system's earlier chunks, which the binning counted),
+//   3. scatter participants into cell order,
+//   4. renumber: slot = first slot of the cell + rank by participant index in
+//      the cell (spatially coherent slots that depend on the cells alone),
+//   5. build each slot's partner list from the 27 neighbouring cells with the
+//      reference's membership test, evaluated in FP64 without contraction:
 //      has_interaction (i < j of a leading participant, not excluded) and
-//      |adjust_direction(r_i, r_j)|^2 < (cutoff (1 + margin))^2.
+//      |adjust_direction(r_i, r_j)|^2 < (cutoff (1 + margin))^2,
+//   6. clear the counters for the next rebuild.
 // The lists hold both directions of every pair (full lists); a pair (a, b) is
 // present iff the reference's half list holds (min(a,b), max(a,b)).
+// The cell counters and chunk sums are zero between rebuilds.
+//
+// The launches before the build are bounded by latency, a few microseconds
+// each: what helps is fewer of them and no serial chain in any.
 #include "list_build.cuh"
 
 namespace mjg {
@@ -28,43 +34,35 @@ namespace {
 constexpr int TPB = 256;
 constexpr int CHUNK = 256;          // items per work chunk
 constexpr int GRID = 148 * 8;       // persistent grid: 8 blocks of 256 per SM
-constexpr int SCAN_TPB = 1024;
+constexpr int CLEAR_GRID = 148;     // the clearing launch: its last block finishes the rebuild
 
-// work counters in t.work: [0] participant chunks, [1] cell chunks, [2] flagged systems
+// work counters in t.work: [0] participant chunks, [1] cell chunks, [3] blocks of the last launch done
 
-__global__ void k_plan(Arena a, int g, TermArrays t, int force_all)
+// one block per system
+__global__ void __launch_bounds__(128) k_plan(Arena a, int g, TermArrays t, int force_all)
 {
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if(s >= a.nsys) {return;}
+    const int s = blockIdx.x;
     GlobalParams& G = a.sys[s].g[g];
-    if(!G.on) {return;}
-    if(force_all) {G.rebuild = 1;}
-    if(!G.rebuild) {return;}
+    if(!G.on || !(force_all || G.rebuild)) {return;}
     const int np = (G.nslot + CHUNK - 1) / CHUNK;
-    const int nc = (G.ncell + CHUNK - 1) / CHUNK;
-    const int bp = atomicAdd(&t.work[0], np);
-    const int bc = atomicAdd(&t.work[1], nc);
-    t.flagged[atomicAdd(&t.work[2], 1)] = s;
-    for(int k = 0; k < np; ++k)
+    const int nc = (G.ncell + CELL_CHUNK - 1) / CELL_CHUNK;
+    __shared__ int base[2];
+    if(threadIdx.x == 0)
+    {
+        G.rebuild = 1;
+        base[0] = atomicAdd(&t.work[0], np);
+        base[1] = atomicAdd(&t.work[1], nc);
+    }
+    __syncthreads();
+    for(int k = threadIdx.x; k < np; k += 128)
     {
         const int b = G.slot_off + k * CHUNK;
-        t.part_chunks[bp + k] = make_int4(s, b, min(b + CHUNK, G.slot_off + G.nslot), 0);
+        t.part_chunks[base[0] + k] = make_int4(s, b, min(b + CHUNK, G.slot_off + G.nslot), 0);
     }
-    for(int k = 0; k < nc; ++k)
+    for(int k = threadIdx.x; k < nc; k += 128)
     {
-        const int b = G.cell_off + k * CHUNK;
-        t.cell_chunks[bc + k] = make_int4(s, b, min(b + CHUNK, G.cell_off + G.ncell), 0);
-    }
-}
-
-__global__ void __launch_bounds__(TPB) k_cells_zero(TermArrays t)
-{
-    const int n = t.work[1];
-    for(int c = blockIdx.x; c < n; c += gridDim.x)
-    {
-        const int4 w = t.cell_chunks[c];
-        const int cell = w.y + threadIdx.x;
-        if(cell < w.z) {t.cell_count[cell] = 0; t.cell_fill[cell] = 0;}
+        const int b = G.cell_off + k * CELL_CHUNK;
+        t.cell_chunks[base[1] + k] = make_int4(s, b, min(b + CELL_CHUNK, G.cell_off + G.ncell), k);
     }
 }
 
@@ -76,155 +74,77 @@ __global__ void __launch_bounds__(TPB) k_cells_assign(Arena a, int g, TermArrays
         const int4 w = t.part_chunks[c];
         const int p = w.y + threadIdx.x;      // participant index (same range as slots)
         if(p >= w.z) {continue;}
-        const GlobalParams& G = a.sys[w.x].g[g];
-        const double4 r = a.pos[t.part_particle[p]];
-        const int cx = cell_coord(r.x, G, 0);
-        const int cy = cell_coord(r.y, G, 1);
-        const int cz = cell_coord(r.z, G, 2);
-        const int cell = G.cell_off + cx + G.dims[0] * (cy + G.dims[1] * cz);
-        t.part_cell[p] = cell;
-        atomicAdd(&t.cell_count[cell], 1);
+        bin_participant(a, t, w.x, a.sys[w.x].g[g], p);
     }
 }
 
-// exclusive scan of one flagged system's cells per block (SCAN_ITEMS cells
-// per thread and pass); cell_start of the system's first cell is its first
-// slot
-constexpr int SCAN_ITEMS = 4;
-__global__ void __launch_bounds__(SCAN_TPB) k_scan_sys(Arena a, int g, TermArrays t)
+// cell_start of one chunk of cells per block and pass, SCAN_ITEMS cells per thread
+constexpr int SCAN_ITEMS = CELL_CHUNK / TPB;
+__global__ void __launch_bounds__(TPB) k_scan_cells(Arena a, int g, TermArrays t)
 {
-    const int nf = t.work[2];
-    __shared__ int warp_tot[SCAN_TPB / 32];
+    const int n = t.work[1];
+    __shared__ int warp_tot[TPB / 32];
     __shared__ int carry;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    for(int f = blockIdx.x; f < nf; f += gridDim.x)
+    for(int c = blockIdx.x; c < n; c += gridDim.x)
     {
-        const GlobalParams& G = a.sys[t.flagged[f]].g[g];
-        if(threadIdx.x == 0) {carry = G.slot_off;}
-        __syncthreads();
-        for(int base = 0; base < G.ncell; base += SCAN_TPB * SCAN_ITEMS)
+        const int4 ch = t.cell_chunks[c];
+        const GlobalParams& G = a.sys[ch.x].g[g];
+        int before = 0;
+        for(int k = threadIdx.x; k < ch.w; k += TPB) {before += t.cell_sum[chunk_sum_index(ch.x, G, k)];}
+        before = __reduce_add_sync(0xffffffffu, before);
+        const int first = ch.y + threadIdx.x * SCAN_ITEMS;     // this thread's cells
+        int v[SCAN_ITEMS];
+        int sum = 0;
+#pragma unroll
+        for(int q = 0; q < SCAN_ITEMS; ++q)
         {
-            const int first = base + threadIdx.x * SCAN_ITEMS;     // this thread's cells
-            int v[SCAN_ITEMS];
-            int sum = 0;
-#pragma unroll
-            for(int q = 0; q < SCAN_ITEMS; ++q)
-            {
-                v[q] = first + q < G.ncell ? t.cell_count[G.cell_off + first + q] : 0;
-                sum += v[q];
-            }
-            int incl = sum;
-#pragma unroll
-            for(int o = 1; o < 32; o <<= 1)
-            {
-                const int y = __shfl_up_sync(0xffffffffu, incl, o);
-                if(lane >= o) {incl += y;}
-            }
-            if(lane == 31) {warp_tot[w] = incl;}
-            __syncthreads();
-            if(w == 0)
-            {
-                const int x = warp_tot[lane];
-                int xi = x;
-#pragma unroll
-                for(int o = 1; o < 32; o <<= 1)
-                {
-                    const int y = __shfl_up_sync(0xffffffffu, xi, o);
-                    if(lane >= o) {xi += y;}
-                }
-                warp_tot[lane] = xi - x;
-            }
-            __syncthreads();
-            int run = carry + warp_tot[w] + incl - sum;
-#pragma unroll
-            for(int q = 0; q < SCAN_ITEMS; ++q)
-            {
-                if(first + q < G.ncell) {t.cell_start[G.cell_off + first + q] = run;}
-                run += v[q];
-            }
-            __syncthreads();
-            if(threadIdx.x == SCAN_TPB - 1) {carry = run;}
-            __syncthreads();
+            v[q] = first + q < ch.z ? t.cell_count[first + q] : 0;
+            sum += v[q];
         }
+        int incl = sum;
+#pragma unroll
+        for(int o = 1; o < 32; o <<= 1)
+        {
+            const int y = __shfl_up_sync(0xffffffffu, incl, o);
+            if(lane >= o) {incl += y;}
+        }
+        if(threadIdx.x == 0) {carry = G.slot_off;}
+        if(lane == 31) {warp_tot[w] = incl;}
+        __syncthreads();
+        if(lane == 0 && before) {atomicAdd(&carry, before);}
+        __syncthreads();
+        int run = carry + incl - sum;
+        for(int k = 0; k < w; ++k) {run += warp_tot[k];}
+#pragma unroll
+        for(int q = 0; q < SCAN_ITEMS; ++q)
+        {
+            if(first + q < ch.z) {t.cell_start[first + q] = run;}
+            run += v[q];
+        }
+        __syncthreads();
     }
 }
 
-__global__ void __launch_bounds__(TPB) k_cells_scatter(TermArrays t, int* slot_tmp)
+__global__ void __launch_bounds__(TPB) k_cells_scatter(TermArrays t)
 {
     const int n = t.work[0];
     for(int c = blockIdx.x; c < n; c += gridDim.x)
     {
         const int4 w = t.part_chunks[c];
         const int p = w.y + threadIdx.x;
-        if(p >= w.z) {continue;}
-        const int cell = t.part_cell[p];
-        const int k = atomicAdd(&t.cell_fill[cell], 1);
-        slot_tmp[t.cell_start[cell] + k] = p;
+        if(p < w.z) {scatter_participant(t, p);}
     }
 }
 
-// rank sort of each cell's members by participant index, so that the slot
-// order depends only on the cell assignment.  A warp takes 32 cells: each
-// lane sorts a small cell (up to SMALL members) by itself, then the warp sorts
-// the larger ones together, one after the other.
-constexpr int SMALL = 8;
-__global__ void __launch_bounds__(TPB) k_cells_sort(TermArrays t, const int* slot_tmp)
-{
-    const int n = t.work[1];
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    const unsigned full = 0xffffffffu;
-    for(int c = blockIdx.x; c < n; c += gridDim.x)
-    {
-        const int4 w = t.cell_chunks[c];
-        for(int cb = w.y + wid * 32; cb < w.z; cb += TPB)
-        {
-            const int cell = cb + lane;
-            int b = 0, m = 0;
-            if(cell < w.z) {b = t.cell_start[cell]; m = t.cell_count[cell];}
-            if(m <= SMALL)
-            {
-                for(int e = 0; e < m; ++e)
-                {
-                    const int v = slot_tmp[b + e];
-                    int rank = 0;
-                    for(int u = 0; u < m; ++u) {rank += slot_tmp[b + u] < v ? 1 : 0;}
-                    t.slot_part[b + rank] = v;
-                }
-            }
-            unsigned big = __ballot_sync(full, m > SMALL);
-            while(big)
-            {
-                const int src = __ffs(big) - 1;
-                big &= big - 1;
-                const int bb = __shfl_sync(full, b, src), mm = __shfl_sync(full, m, src);
-                for(int e = lane; e < mm; e += 32)
-                {
-                    const int v = slot_tmp[bb + e];
-                    int rank = 0;
-                    for(int u = 0; u < mm; ++u) {rank += slot_tmp[bb + u] < v ? 1 : 0;}
-                    t.slot_part[bb + rank] = v;
-                }
-            }
-        }
-    }
-}
-
-__global__ void __launch_bounds__(TPB) k_slots_setup(Arena a, TermArrays t)
+__global__ void __launch_bounds__(TPB) k_slots_place(Arena a, TermArrays t)
 {
     const int n = t.work[0];
     for(int c = blockIdx.x; c < n; c += gridDim.x)
     {
         const int4 w = t.part_chunks[c];
-        const int s = w.y + threadIdx.x;
-        if(s >= w.z) {continue;}
-        const int p = t.slot_part[s];
-        const int i = t.part_particle[p];
-        const double4 r = a.pos[i];
-        t.slot_particle[s] = i;
-        t.slot_of[i]       = s;
-        t.slot_sys[s]      = w.x;
-        t.slot_pd[s]       = make_double4(r.x, r.y, r.z, t.part_p0[p]);
-        if(t.part_p1) {t.slot_p1[s] = t.part_p1[p];}
+        const int p = w.y + threadIdx.x;
+        if(p < w.z) {place_participant(a, t, w.x, p);}
     }
 }
 
@@ -255,10 +175,23 @@ __global__ void __launch_bounds__(TPB) k_build_list(Arena a, int g, TermArrays t
     }
 }
 
-__global__ void k_rebuild_done(Arena a, int g, TermArrays t, int forced)
+// clears the rebuilt systems' cell counters and chunk sums, then (the last
+// block to finish) their flags and the work lists
+__global__ void __launch_bounds__(TPB) k_rebuild_done(Arena a, int g, TermArrays t, int forced)
 {
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if(s < a.nsys)
+    const int n = t.work[1];
+    for(int c = blockIdx.x; c < n; c += gridDim.x)
+    {
+        const int4 ch = t.cell_chunks[c];
+        for(int cell = ch.y + threadIdx.x; cell < ch.z; cell += TPB) {t.cell_count[cell] = 0;}
+        if(threadIdx.x == 0) {t.cell_sum[chunk_sum_index(ch.x, a.sys[ch.x].g[g], ch.w)] = 0;}
+    }
+    __shared__ bool last;
+    __syncthreads();
+    if(threadIdx.x == 0) {last = atomicAdd(&t.work[3], 1) == (int)gridDim.x - 1;}
+    __syncthreads();
+    if(!last) {return;}
+    for(int s = threadIdx.x; s < a.nsys; s += TPB)
     {
         GlobalParams& G = a.sys[s].g[g];
         if(G.on && G.rebuild)
@@ -268,7 +201,8 @@ __global__ void k_rebuild_done(Arena a, int g, TermArrays t, int forced)
             if(!forced) {G.rebuilds += 1;}   // count only reduce_margin rebuilds
         }
     }
-    if(s == 0) {t.work[0] = 0; t.work[1] = 0; t.work[2] = 0; *t.any_rebuild = 0;}
+    if(threadIdx.x < 4) {t.work[threadIdx.x] = 0;}
+    if(threadIdx.x == 0) {*t.any_rebuild = 0;}
 }
 
 __global__ void k_scatter_param(TermArrays t, double* w)
@@ -306,19 +240,17 @@ void launch_sum_counts(const TermArrays& t, cudaStream_t s)
 void launch_rebuild(const Arena& a, int g, TermArrays& t, int force_all, cudaStream_t s)
 {
     if(!t.on || t.np == 0) {return;}
-    k_plan        <<<blocks(a.nsys, 128), 128, 0, s>>>(a, g, t, force_all);
-    k_cells_zero  <<<GRID, TPB, 0, s>>>(t);
-    k_cells_assign<<<GRID, TPB, 0, s>>>(a, g, t);
-    k_scan_sys    <<<min(a.nsys, 1024), SCAN_TPB, 0, s>>>(a, g, t);
-    k_cells_scatter<<<GRID, TPB, 0, s>>>(t, t.slot_particle);
-    k_cells_sort  <<<GRID, TPB, 0, s>>>(t, t.slot_particle);
-    k_slots_setup <<<GRID, TPB, 0, s>>>(a, t);
+    k_plan         <<<a.nsys, 128, 0, s>>>(a, g, t, force_all);
+    k_cells_assign <<<GRID, TPB, 0, s>>>(a, g, t);
+    k_scan_cells   <<<GRID, TPB, 0, s>>>(a, g, t);
+    k_cells_scatter<<<GRID, TPB, 0, s>>>(t);
+    k_slots_place  <<<GRID, TPB, 0, s>>>(a, t);
     if(t.build_lanes == 4)       {k_build_list<4> <<<GRID, TPB, 0, s>>>(a, g, t);}
     else if(t.build_lanes == 8)  {k_build_list<8> <<<GRID, TPB, 0, s>>>(a, g, t);}
     else if(t.build_lanes == 16) {k_build_list<16><<<GRID, TPB, 0, s>>>(a, g, t);}
     else                         {k_build_list<32><<<GRID, TPB, 0, s>>>(a, g, t);}
-    k_rebuild_done<<<blocks(a.nsys, 128), 128, 0, s>>>(a, g, t, force_all);
-    note_launches(9);
+    k_rebuild_done <<<CLEAR_GRID, TPB, 0, s>>>(a, g, t, force_all);
+    note_launches(7);
 }
 
 }  // namespace mjg

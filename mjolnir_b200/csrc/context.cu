@@ -132,7 +132,7 @@ struct HostSystem {
 
 struct TermDev {
     DevBuf part_particle, part_p0, part_p1, part_sys, part_cell;
-    DevBuf cell_count, cell_start, cell_fill, work, part_chunks, cell_chunks, flagged;
+    DevBuf cell_count, cell_start, cell_sum, work, part_chunks, cell_chunks;
     DevBuf slot_part, slot_particle, slot_sys, slot_pd, slot_p1, slot_of, slot_w;
     DevBuf nnb, nbr, max_count, any_rebuild;
     DevBuf ex_start, ex_idx;
@@ -218,8 +218,8 @@ int64_t device_bytes(const mjg_context* c)
     for(const auto& t : c->term)
     {
         const DevBuf* tb[] = {&t.part_particle, &t.part_p0, &t.part_p1, &t.part_sys,
-                              &t.part_cell, &t.cell_count, &t.cell_start, &t.cell_fill,
-                              &t.work, &t.part_chunks, &t.cell_chunks, &t.flagged, &t.slot_part, &t.slot_particle,
+                              &t.part_cell, &t.cell_count, &t.cell_start, &t.cell_sum,
+                              &t.work, &t.part_chunks, &t.cell_chunks, &t.slot_part, &t.slot_particle,
                               &t.slot_sys, &t.slot_pd, &t.slot_p1, &t.slot_of, &t.slot_w, &t.nnb, &t.nbr, &t.max_count,
                               &t.any_rebuild, &t.ex_start, &t.ex_idx};
         for(auto* x : tb) {b += (int64_t)x->cap;}
@@ -1169,8 +1169,8 @@ void commit(mjg_context* c)
         if(!t.on)
         {
             DevBuf* bufs[] = {&T.part_particle, &T.part_p0, &T.part_p1, &T.part_sys,
-                              &T.part_cell, &T.cell_count, &T.cell_start, &T.cell_fill,
-                              &T.work, &T.part_chunks, &T.cell_chunks, &T.flagged, &T.slot_part, &T.slot_particle,
+                              &T.part_cell, &T.cell_count, &T.cell_start, &T.cell_sum,
+                              &T.work, &T.part_chunks, &T.cell_chunks, &T.slot_part, &T.slot_particle,
                               &T.slot_sys, &T.slot_pd, &T.slot_p1, &T.slot_of, &T.slot_w, &T.nnb, &T.nbr,
                               &T.max_count, &T.any_rebuild};
             for(auto* b : bufs) {b->release();}
@@ -1183,22 +1183,15 @@ void commit(mjg_context* c)
         put(T.part_sys, c_ps[g]);
         T.part_cell.ensure(sizeof(int) * np);
         T.cell_count.ensure(sizeof(int) * t.ncell);
-        T.cell_fill.ensure(sizeof(int) * t.ncell);
-        T.cell_start.ensure(sizeof(int) * (t.ncell + 1));
+        T.cell_sum.ensure(sizeof(int) * t.ncell);
+        T.cell_start.ensure(sizeof(int) * t.ncell);
         // rebuild work lists (sized for every system flagged at once)
         T.work.ensure(sizeof(int) * 4);
         CK(cudaMemsetAsync(T.work.p, 0, T.work.bytes, st));
         T.part_chunks.ensure(sizeof(int4) * std::max<long long>(1, part_chunk_cap[g]));
         T.cell_chunks.ensure(sizeof(int4) * std::max<long long>(1, cell_chunk_cap[g]));
-        T.flagged.ensure(sizeof(int) * std::max(1, nsys));
-        {
-            const int last = (int)np;        // cell_start[ncell] = total slots
-            CK(cudaMemcpyAsync(T.cell_start.as<int>() + t.ncell, &last, sizeof(int),
-                               cudaMemcpyHostToDevice, st));
-            CK(cudaStreamSynchronize(st));
-        }
         CK(cudaMemsetAsync(T.cell_count.p, 0, T.cell_count.bytes, st));
-        CK(cudaMemsetAsync(T.cell_fill.p, 0, T.cell_fill.bytes, st));
+        CK(cudaMemsetAsync(T.cell_sum.p, 0, T.cell_sum.bytes, st));
         T.slot_part.ensure(sizeof(int) * np);
         T.slot_particle.ensure(sizeof(int) * np);
         T.slot_sys.ensure(sizeof(int) * np);
@@ -1219,11 +1212,10 @@ void commit(mjg_context* c)
         t.part_cell = T.part_cell.as<int>();
         t.cell_count = T.cell_count.as<int>();
         t.cell_start = T.cell_start.as<int>();
-        t.cell_fill = T.cell_fill.as<int>();
+        t.cell_sum = T.cell_sum.as<int>();
         t.work = T.work.as<int>();
         t.part_chunks = T.part_chunks.as<int4>();
         t.cell_chunks = T.cell_chunks.as<int4>();
-        t.flagged = T.flagged.as<int>();
         t.slot_part = T.slot_part.as<int>();
         t.slot_particle = T.slot_particle.as<int>();
         t.slot_sys = T.slot_sys.as<int>();
@@ -1574,7 +1566,7 @@ void mjg_context_destroy(mjg_context* c)
     for(auto& t : c->term)
     {
         DevBuf* bufs[] = {&t.part_particle, &t.part_p0, &t.part_p1, &t.part_sys,
-                          &t.part_cell, &t.cell_count, &t.cell_start, &t.cell_fill, &t.work, &t.part_chunks, &t.cell_chunks, &t.flagged,
+                          &t.part_cell, &t.cell_count, &t.cell_start, &t.cell_sum, &t.work, &t.part_chunks, &t.cell_chunks,
                           &t.slot_part, &t.slot_particle, &t.slot_sys, &t.slot_pd,
                           &t.slot_p1, &t.slot_of, &t.slot_w, &t.nnb, &t.nbr, &t.max_count, &t.any_rebuild, &t.ex_start,
                           &t.ex_idx};

@@ -63,13 +63,12 @@ struct TermArrays {
     const double* part_p1;      // [np] LJ epsilon
     const int* part_sys;        // [np]
     int*       part_cell;       // [np]
-    int*       cell_count;      // [ncell]
-    int*       cell_start;      // [ncell + 1]
-    int*       cell_fill;       // [ncell]
-    int*       work;            // [3] rebuild work counters
+    int*       cell_count;      // [ncell] zero between rebuilds
+    int*       cell_start;      // [ncell]
+    int*       cell_sum;        // [ncell] participants per chunk of cells (chunk_sum_index), zero between rebuilds
+    int*       work;            // [4] rebuild work counters
     int4*      part_chunks;     // rebuild work: participant chunks {sys, begin, end}
     int4*      cell_chunks;     // rebuild work: cell chunks
-    int*       flagged;         // [nsys] systems rebuilding this step
     int*       slot_part;       // [np] scratch of the rebuild: participants in cell order, then list lengths
     int*       slot_particle;   // [np] global particle of slot
     int*       slot_sys;        // [np]

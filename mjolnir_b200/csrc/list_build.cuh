@@ -1,9 +1,58 @@
-// The Verlet list of one slot, shared by the rebuild's list build launches
-// (cells.cu) and the multi-step kernel of small arenas (run.cu).
+// The parts of a list rebuild that work on one participant or one slot, shared
+// by the rebuild's launches (cells.cu) and the multi-step kernel of small arenas (run.cu).
 #pragma once
 #include "kernels.cuh"
 
 namespace mjg {
+
+constexpr int CELL_CHUNK = 1024;     // cells per scan item
+
+// A system's chunk sums lie where its cells do, one word per chunk: chunk k's at
+// cell cell_off + k.
+__device__ __forceinline__ int chunk_sum_index(int, const GlobalParams& G, int k) {return G.cell_off + k;}
+
+// Bins participant p of the system: its cell and its place in the cell; counts
+// the cell and the cell's chunk (one atomic per chunk and warp; the only chunk of
+// a small grid is never summed up).
+__device__ __forceinline__ void bin_participant(const Arena& a, const TermArrays& t, int sys, const GlobalParams& G, int p)
+{
+    const double4 r = a.pos[t.part_particle[p]];
+    const int c = cell_coord(r.x, G, 0) + G.dims[0] * (cell_coord(r.y, G, 1) + G.dims[1] * cell_coord(r.z, G, 2));
+    t.part_cell[p] = G.cell_off + c;
+    t.nnb[p] = atomicAdd(&t.cell_count[G.cell_off + c], 1);    // scratch until the build writes the lengths
+    if(G.ncell > CELL_CHUNK)
+    {
+        const int chunk = chunk_sum_index(sys, G, c / CELL_CHUNK);
+        const unsigned same = __match_any_sync(__activemask(), chunk);
+        if((threadIdx.x & 31) == __ffs(same) - 1) {atomicAdd(&t.cell_sum[chunk], __popc(same));}
+    }
+}
+
+// participants in cell order, in any order within a cell
+__device__ __forceinline__ void scatter_participant(const TermArrays& t, int p)
+{
+    t.slot_part[t.cell_start[t.part_cell[p]] + t.nnb[p]] = p;
+}
+
+// Participant p's slot, its rank by participant index within its cell (so that
+// the slot order depends only on the cell assignment), and the slot's entries.
+// A thread per participant ranks against the whole cell: a cell of m members
+// costs each m loads in parallel, where sorting a cell by one lane or warp made
+// one long chain of it (cells of 45 members: 187 us, now 6).
+__device__ __forceinline__ void place_participant(const Arena& a, const TermArrays& t, int sys, int p)
+{
+    const int c = t.part_cell[p];
+    const int i = t.part_particle[p];
+    const int b = t.cell_start[c], m = t.cell_count[c];
+    const double4 r = a.pos[i];
+    int slot = b;
+    for(int u = 0; u < m; ++u) {slot += t.slot_part[b + u] < p ? 1 : 0;}
+    t.slot_particle[slot] = i;
+    t.slot_of[i]          = slot;
+    t.slot_sys[slot]      = sys;
+    t.slot_pd[slot]       = make_double4(r.x, r.y, r.z, t.part_p0[p]);
+    if(t.part_p1) {t.slot_p1[slot] = t.part_p1[p];}
+}
 
 // A slot's exclusion row staged in shared memory once per slot: the CSR row of
 // particle i holds every particle excluded together with i (the relation is

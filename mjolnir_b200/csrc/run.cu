@@ -36,7 +36,7 @@ namespace {
 
 constexpr int RT = 1024;                 // threads per block
 constexpr int RUN_BATCH = 2;             // partners a thread requests together
-constexpr int CELL_CHUNK = RT;           // cells per scan item
+static_assert(CELL_CHUNK == RT, "one cell per thread of a scan item");
 
 using ull = unsigned long long;
 
@@ -122,7 +122,6 @@ __device__ __forceinline__ void add_force(void* force, long long i, const Acc<P_
 // (dynamic; the arena's pointer is replaced by it), read by every phase without
 // a trip to L2; the remaining skins are kept there by every block for itself.
 struct Shared {
-    int chunk_off[RUN_MAX_SYSTEMS][NGLOBAL];     // first chunk sum of each system
     int rebuilds[RUN_MAX_SYSTEMS][NGLOBAL];
     ull flag[NGLOBAL];                           // systems to rebuild, a bit each
     int scan[32];
@@ -178,14 +177,12 @@ __device__ __forceinline__ void build(const Arena& a, int g, const TermArrays& t
 }
 
 // The lists of the flagged systems of term g at the current positions.  The
-// cell counters and chunk sums are zero on entry (the force phase that follows
-// each rebuild clears them).
+// cell counters and chunk sums are zero on entry (cells.cu); the force phase that
+// follows each rebuild clears them.
 template<int g>
 __device__ __forceinline__ bool rebuild(const Arena& a, const TermArrays& t, ull mask, const Grid& G, Shared& sh,
                                         Barrier& bar)
 {
-    int* const csum = reinterpret_cast<int*>(t.cell_chunks);
-    int* const rank = t.nnb;                 // scratch until the build writes the lengths
     auto nslot = [&](int s) {return a.sys[s].g[g].nslot;};
     int k, s = 0;
     // bin the participants; each takes its place within its cell
@@ -194,17 +191,7 @@ __device__ __forceinline__ bool rebuild(const Arena& a, const TermArrays& t, ull
         k = e;
         if(!locate(mask, k, s, nslot)) {break;}
         const GlobalParams& P = a.sys[s].g[g];
-        const int p = P.slot_off + k;
-        const double4 x = a.pos[t.part_particle[p]];
-        const int c = cell_coord(x.x, P, 0) + P.dims[0] * (cell_coord(x.y, P, 1) + P.dims[1] * cell_coord(x.z, P, 2));
-        t.part_cell[p] = P.cell_off + c;
-        rank[p] = atomicAdd(&t.cell_count[P.cell_off + c], 1);
-        if(P.ncell > CELL_CHUNK)                 // a single chunk's sum is not read
-        {
-            const int chunk = sh.chunk_off[s][g] + c / CELL_CHUNK;
-            const unsigned same = __match_any_sync(__activemask(), chunk);
-            if((threadIdx.x & 31) == __ffs(same) - 1) {atomicAdd(&csum[chunk], __popc(same));}
-        }
+        bin_participant(a, t, s, P, P.slot_off + k);
     }
     if(!bar.sync()) {return false;}
     // first slot of each cell: one block per chunk of cells; the sums of the
@@ -216,7 +203,7 @@ __device__ __forceinline__ bool rebuild(const Arena& a, const TermArrays& t, ull
         if(!locate(mask, k, s, [&](int x) {return (a.sys[x].g[g].ncell + CELL_CHUNK - 1) / CELL_CHUNK;})) {break;}
         const GlobalParams& q = a.sys[s].g[g];
         int before = 0;
-        for(int c = threadIdx.x; c < k; c += RT) {before += csum[sh.chunk_off[s][g] + c];}
+        for(int c = threadIdx.x; c < k; c += RT) {before += t.cell_sum[chunk_sum_index(s, q, c)];}
         before = __reduce_add_sync(0xffffffffu, before);
         const int cell = k * CELL_CHUNK + threadIdx.x;
         const int v = cell < q.ncell ? t.cell_count[q.cell_off + cell] : 0;
@@ -254,28 +241,14 @@ __device__ __forceinline__ bool rebuild(const Arena& a, const TermArrays& t, ull
     {
         k = e;
         if(!locate(mask, k, s, nslot)) {break;}
-        const int p = a.sys[s].g[g].slot_off + k;
-        t.slot_part[t.cell_start[t.part_cell[p]] + rank[p]] = p;
+        scatter_participant(t, a.sys[s].g[g].slot_off + k);
     }
     if(!bar.sync()) {return false;}
-    // each participant's slot: its rank by participant index within its cell,
-    // so that the slot order depends only on the cell assignment
     for(int e = G.thread;; e += G.nthread)
     {
         k = e;
         if(!locate(mask, k, s, nslot)) {break;}
-        const int p = a.sys[s].g[g].slot_off + k;
-        const int c = t.part_cell[p];
-        const int b = t.cell_start[c], m = t.cell_count[c];
-        const int i = t.part_particle[p];
-        const double4 x = a.pos[i];
-        int slot = b;
-        for(int u = 0; u < m; ++u) {slot += t.slot_part[b + u] < p ? 1 : 0;}
-        t.slot_particle[slot] = i;
-        t.slot_of[i]          = slot;
-        t.slot_sys[slot]      = s;
-        t.slot_pd[slot]       = make_double4(x.x, x.y, x.z, t.part_p0[p]);
-        if(t.part_p1) {t.slot_p1[slot] = t.part_p1[p];}
+        place_participant(a, t, s, a.sys[s].g[g].slot_off + k);
     }
     if(!bar.sync()) {return false;}
     // narrow groups for short candidate sequences, as the launched build
@@ -285,8 +258,7 @@ __device__ __forceinline__ bool rebuild(const Arena& a, const TermArrays& t, ull
 }
 
 // clears the flagged systems' cell counters and chunk sums for the next rebuild
-__device__ __forceinline__ void clear_cells(const Arena& a, const TermArrays& t, int g, ull mask, const Grid& G,
-                                            const Shared& sh)
+__device__ __forceinline__ void clear_cells(const Arena& a, const TermArrays& t, int g, ull mask, const Grid& G)
 {
     for(ull m = mask; m; m &= m - 1)
     {
@@ -294,7 +266,7 @@ __device__ __forceinline__ void clear_cells(const Arena& a, const TermArrays& t,
         const GlobalParams& q = a.sys[s].g[g];
         for(int c = G.thread; c < q.ncell; c += G.nthread) {t.cell_count[q.cell_off + c] = 0;}
         const int nc = (q.ncell + CELL_CHUNK - 1) / CELL_CHUNK;
-        for(int c = G.thread; c < nc; c += G.nthread) {reinterpret_cast<int*>(t.cell_chunks)[sh.chunk_off[s][g] + c] = 0;}
+        for(int c = G.thread; c < nc; c += G.nthread) {t.cell_sum[chunk_sum_index(s, q, c)] = 0;}
     }
 }
 
@@ -430,23 +402,6 @@ __global__ void __launch_bounds__(RT, 1) k_run(const __grid_constant__ RunArgs r
         for(int w = threadIdx.x; w < nsys * NGLOBAL; w += RT) {(&sh.rebuilds[0][0])[w] = 0;}
     }
     __syncthreads();
-    if(threadIdx.x < NGLOBAL)
-    {
-        int c = 0;
-        for(int s = 0; s < nsys; ++s)
-        {
-            sh.chunk_off[s][threadIdx.x] = c;
-            c += (sys[s].g[threadIdx.x].ncell + CELL_CHUNK - 1) / CELL_CHUNK;
-        }
-    }
-    __syncthreads();
-    for(int g = 0; g < NGLOBAL; ++g)
-    {
-        if(!r.t[g].on) {continue;}
-        for(int c = G.thread; c < r.t[g].ncell; c += G.nthread) {r.t[g].cell_count[c] = 0;}
-        const int nc = sh.chunk_off[nsys - 1][g] + (sys[nsys - 1].g[g].ncell + CELL_CHUNK - 1) / CELL_CHUNK;
-        for(int c = G.thread; c < nc; c += G.nthread) {reinterpret_cast<int*>(r.t[g].cell_chunks)[c] = 0;}
-    }
     ull* const disp = r.disp2;                    // [2][nsys], zero between launches
 
     // this thread's first particle and its noise, drawn while the grid waits
@@ -517,7 +472,7 @@ __global__ void __launch_bounds__(RT, 1) k_run(const __grid_constant__ RunArgs r
         if(sh.flag[G_LJ] && !rebuild<G_LJ>(a, r.t[G_LJ], sh.flag[G_LJ], G, sh, bar)) {return;}
         // ---- forces
         forces<PREC>(a, r, G);
-        for(int g = 0; g < NGLOBAL; ++g) {if(sh.flag[g]) {clear_cells(a, r.t[g], g, sh.flag[g], G, sh);}}
+        for(int g = 0; g < NGLOBAL; ++g) {if(sh.flag[g]) {clear_cells(a, r.t[g], g, sh.flag[g], G);}}
         bar.arrive();
         draw(k + 1);                              // while the others finish
         if(!bar.wait()) {return;}
