@@ -31,12 +31,12 @@ constexpr int TPB = 256;
 template<int PREC, bool NF, bool NE>
 __global__ void __launch_bounds__(TPB, PREC == P_MIXED ? 5 : 3) k_local(Arena a, LocalArrays l, int mask)
 {
-    __shared__ typename WinT<PREC>::type win[3 * WINDOW];
+    __shared__ typename WinT<PREC>::type win[Window<PREC>::SIZE];
     const int w = blockIdx.x;
     Window<PREC> W{win, w * SEG};
     if(NF)
     {
-        for(int k = threadIdx.x; k < 3 * WINDOW; k += TPB) {win[k] = 0;}
+        for(int k = threadIdx.x; k < Window<PREC>::SIZE; k += TPB) {win[k] = 0;}
         __syncthreads();
     }
     if(mask & 1)

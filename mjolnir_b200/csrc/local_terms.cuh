@@ -14,15 +14,29 @@ constexpr int SEG = 256;              // particles owned by one block (window st
 constexpr int HALO = 64;              // terms may reach this far past the window
 constexpr int WINDOW = SEG + HALO;
 
+// FP64 sums in the plain form.  The mixed form's 64-bit integer sums are kept as
+// two 32-bit words each: shared memory adds 32-bit words in one instruction and
+// 64-bit ones in a compare-and-swap loop.  The low word's add returns what it
+// found, which gives the carry, and the high word is touched only where it
+// changes.
 template<int PREC> struct WinT;
-template<> struct WinT<P_FP64>  {using type = double;};
-template<> struct WinT<P_MIXED> {using type = unsigned long long;};
+template<> struct WinT<P_FP64>  {using type = double; static constexpr int words = 1;};
+template<> struct WinT<P_MIXED> {using type = unsigned; static constexpr int words = 2;};
 
 template<int PREC>
 struct Window {
     using T = typename WinT<PREC>::type;
-    T* w;         // [3 * WINDOW] in shared memory
+    static constexpr int SIZE = 3 * WINDOW * WinT<PREC>::words;
+    T* w;         // [SIZE] in shared memory; mixed: low words, then high words
     int base;
+    __device__ __forceinline__ void add64(int k, long long v)
+    {
+        unsigned* lo = reinterpret_cast<unsigned*>(w) + k;
+        const unsigned l = (unsigned)v;
+        const unsigned old = atomicAdd(lo, l);
+        const unsigned h = (unsigned)((unsigned long long)v >> 32) + (old + l < l ? 1u : 0u);
+        if(h) {atomicAdd(lo + 3 * WINDOW, h);}
+    }
     __device__ __forceinline__ void add(void* force, int i, double fx, double fy, double fz)
     {
         const int k = i - base;
@@ -36,9 +50,9 @@ struct Window {
             }
             else
             {
-                atomicAdd(reinterpret_cast<unsigned long long*>(w) + 3 * k + 0, (unsigned long long)fx_from_double(fx));
-                atomicAdd(reinterpret_cast<unsigned long long*>(w) + 3 * k + 1, (unsigned long long)fx_from_double(fy));
-                atomicAdd(reinterpret_cast<unsigned long long*>(w) + 3 * k + 2, (unsigned long long)fx_from_double(fz));
+                add64(3 * k + 0, fx_from_double(fx));
+                add64(3 * k + 1, fx_from_double(fy));
+                add64(3 * k + 2, fx_from_double(fz));
             }
             return;
         }
@@ -65,18 +79,23 @@ struct Window {
         {
             const long long i = (long long)base + k;
             if(i >= n) {break;}
-            const T x = w[3 * k], y = w[3 * k + 1], z = w[3 * k + 2];
-            if(x == T(0) && y == T(0) && z == T(0)) {continue;}
             if(PREC == P_FP64)
             {
+                const double* v = reinterpret_cast<const double*>(w) + 3 * k;
+                if(v[0] == 0.0 && v[1] == 0.0 && v[2] == 0.0) {continue;}
                 double* f = reinterpret_cast<double*>(static_cast<double4*>(force) + i);
-                atomicAdd(f + 0, (double)x); atomicAdd(f + 1, (double)y); atomicAdd(f + 2, (double)z);
+                atomicAdd(f + 0, v[0]); atomicAdd(f + 1, v[1]); atomicAdd(f + 2, v[2]);
             }
             else
             {
+                const unsigned* v = reinterpret_cast<const unsigned*>(w) + 3 * k;
                 unsigned long long* f = reinterpret_cast<unsigned long long*>(static_cast<longlong4*>(force) + i);
-                atomicAdd(f + 0, (unsigned long long)x); atomicAdd(f + 1, (unsigned long long)y);
-                atomicAdd(f + 2, (unsigned long long)z);
+#pragma unroll
+                for(int c = 0; c < 3; ++c)
+                {
+                    const unsigned long long x = (unsigned long long)v[3 * WINDOW + c] << 32 | v[c];
+                    if(x) {atomicAdd(f + c, x);}
+                }
             }
         }
     }
