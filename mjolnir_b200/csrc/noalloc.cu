@@ -28,16 +28,19 @@ namespace {
 constexpr int NA_MAX_PARTICLES = 65536;
 constexpr int NA_MAX_CELLS     = 65536;
 constexpr int NA_TPB           = 256;
+constexpr int NA_BLOCKS        = 64;      // blocks of the radius pass
+constexpr int NA_SCAN          = 1024;    // cells per block of the scan
+constexpr int NA_LANES         = 8;       // lanes per particle of the force pass
 
-// header: [0] dims x, [1] dims y, [2] dims z, [3] hashed, [4..5] max radius (double bits)
+// header: [0] dims x, [1] dims y, [2] dims z, [3] hashed
 struct NaScratch {
-    int    header[8];
-    double inv_w;
-    double pad[7];
-    int    count[NA_MAX_CELLS];
-    int    start[NA_MAX_CELLS + 1];
-    int    fill[NA_MAX_CELLS];
-    int    order[NA_MAX_PARTICLES];
+    int      header[8];
+    double   inv_w;
+    double   max_radius[NA_BLOCKS];       // of each block's share
+    int      count[NA_MAX_CELLS];
+    int      start[NA_MAX_CELLS + 1];
+    unsigned place[NA_MAX_PARTICLES];     // cell, and rank within it, 16 bits each
+    int      order[NA_MAX_PARTICLES];
 };
 
 // The one scratch area of this entry point (about 1 MiB per device).  In host
@@ -50,58 +53,69 @@ struct NaBox {
     double lower[3], width[3], halfw[3];
 };
 
-// one block: largest radius, grid shape, counters to zero
-__global__ void k_na_setup(NaScratch* sc, long long n, const double* radius, double cutoff_ratio,
-                           NaBox box, double* energy)
+// The five launches of a call are a few microseconds of latency each: every one
+// spreads its work over the GPU (one block that took the largest radius, cleared
+// 65,536 cells and scanned them took 60 us of a call's 150).
+
+// largest radius of each block's share, counters to zero
+__global__ void __launch_bounds__(NA_TPB) k_na_radius(NaScratch* sc, long long n, const double* radius, double* energy)
 {
-    __shared__ double red[NA_TPB];
+    __shared__ double red[NA_TPB / 32];
+    const int t = blockIdx.x * NA_TPB + threadIdx.x;
     double m = 0.0;
-    for(long long i = threadIdx.x; i < n; i += NA_TPB) {m = fmax(m, radius[i]);}
-    red[threadIdx.x] = m;
+    for(long long i = t; i < n; i += NA_BLOCKS * NA_TPB) {m = fmax(m, radius[i]);}
+#pragma unroll
+    for(int o = 16; o > 0; o >>= 1) {m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));}
+    if((threadIdx.x & 31) == 0) {red[threadIdx.x >> 5] = m;}
+    // the previous call's contents must not leak into this one
+    for(int c = t; c < NA_MAX_CELLS; c += NA_BLOCKS * NA_TPB) {sc->count[c] = 0;}
+    if(t == 0) {*energy = 0.0;}
     __syncthreads();
-    for(int o = NA_TPB / 2; o > 0; o >>= 1)
-    {
-        if(threadIdx.x < o) {red[threadIdx.x] = fmax(red[threadIdx.x], red[threadIdx.x + o]);}
-        __syncthreads();
-    }
     if(threadIdx.x == 0)
     {
-        const double rc = red[0] * 2 * cutoff_ratio;   // ExcludedVolumePotential::max_cutoff
-        int d[3];
-        if(box.periodic)
-        {
-            for(int x = 0; x < 3; ++x)
-            {
-                const double c = rc > 0 ? floor(box.width[x] / rc) : 3.0;
-                d[x] = (int)fmin(fmax(c, 3.0), 64.0);   // at least 3, cells at least rc wide
-            }
-            while((long long)d[0] * d[1] * d[2] > NA_MAX_CELLS)
-            {
-                int b = 0;
-                for(int x = 1; x < 3; ++x) {if(d[x] > d[b]) {b = x;}}
-                d[b] -= 1;
-            }
-            sc->inv_w = 0.0;
-        }
-        else
-        {
-            // unbounded space: cells rc wide hashed modulo a small grid
-            int dd = (int)ceil(cbrt((double)n));
-            dd = dd < 3 ? 3 : (dd > 32 ? 32 : dd);
-            d[0] = d[1] = d[2] = dd;
-            sc->inv_w = rc > 0 ? 1.0 / (rc * (1 + 1e-9)) : 0.0;
-        }
-        sc->header[0] = d[0]; sc->header[1] = d[1]; sc->header[2] = d[2];
-        sc->header[3] = box.periodic ? 0 : 1;
-        *energy = 0.0;
+        for(int k = 1; k < NA_TPB / 32; ++k) {m = fmax(m, red[k]);}
+        sc->max_radius[blockIdx.x] = m;
     }
-    // the previous call's contents must not leak into this one
-    for(int c = threadIdx.x; c < NA_MAX_CELLS; c += NA_TPB) {sc->count[c] = 0; sc->fill[c] = 0;}
 }
 
-__device__ __forceinline__ int na_coord(const NaScratch* sc, const NaBox& box, double x, int axis)
+// grid shape from the largest radius, by every block of the binning for itself
+__device__ __forceinline__ void na_grid(const NaScratch* sc, long long n, double cutoff_ratio, const NaBox& box,
+                                        int (&header)[4], double& inv_w)
 {
-    const int d = sc->header[axis];
+    double mr = 0.0;
+    for(int k = 0; k < NA_BLOCKS; ++k) {mr = fmax(mr, sc->max_radius[k]);}
+    const double rc = mr * 2 * cutoff_ratio;       // ExcludedVolumePotential::max_cutoff
+    int d[3];
+    if(box.periodic)
+    {
+        for(int x = 0; x < 3; ++x)
+        {
+            const double c = rc > 0 ? floor(box.width[x] / rc) : 3.0;
+            d[x] = (int)fmin(fmax(c, 3.0), 64.0);   // at least 3, cells at least rc wide
+        }
+        while((long long)d[0] * d[1] * d[2] > NA_MAX_CELLS)
+        {
+            int b = 0;
+            for(int x = 1; x < 3; ++x) {if(d[x] > d[b]) {b = x;}}
+            d[b] -= 1;
+        }
+        inv_w = 0.0;
+    }
+    else
+    {
+        // unbounded space: cells rc wide hashed modulo a small grid
+        int dd = (int)ceil(cbrt((double)n));
+        dd = dd < 3 ? 3 : (dd > 32 ? 32 : dd);
+        d[0] = d[1] = d[2] = dd;
+        inv_w = rc > 0 ? 1.0 / (rc * (1 + 1e-9)) : 0.0;
+    }
+    header[0] = d[0]; header[1] = d[1]; header[2] = d[2];
+    header[3] = box.periodic ? 0 : 1;
+}
+
+__device__ __forceinline__ int na_coord(const int* header, double inv_w, const NaBox& box, double x, int axis)
+{
+    const int d = header[axis];
     if(box.periodic)
     {
         // wrapped: a particle a little outside [lower, upper) lands in the
@@ -109,100 +123,155 @@ __device__ __forceinline__ int na_coord(const NaScratch* sc, const NaBox& box, d
         long long c = (long long)floor((x - box.lower[axis]) / (box.width[axis] / d)) % d;
         return (int)(c < 0 ? c + d : c);
     }
-    long long c = (long long)floor(x * sc->inv_w) % d;
+    long long c = (long long)floor(x * inv_w) % d;
     return (int)(c < 0 ? c + d : c);
 }
 
-__device__ __forceinline__ int na_cell(const NaScratch* sc, int x, int y, int z)
+// cell of each particle and its place in the cell
+__global__ void __launch_bounds__(NA_TPB) k_na_bin(NaScratch* sc, long long n, const double* pos, double cutoff_ratio, NaBox box)
 {
-    return x + sc->header[0] * (y + sc->header[1] * z);
-}
-
-__global__ void k_na_bin(NaScratch* sc, long long n, const double* pos, NaBox box)
-{
-    const long long i = (long long)blockIdx.x * NA_TPB + threadIdx.x;
-    if(i >= n) {return;}
-    const int c = na_cell(sc, na_coord(sc, box, pos[3 * i], 0), na_coord(sc, box, pos[3 * i + 1], 1),
-                          na_coord(sc, box, pos[3 * i + 2], 2));
-    atomicAdd(&sc->count[c], 1);
-}
-
-// one block: exclusive scan of the cell counts
-__global__ void k_na_scan(NaScratch* sc)
-{
-    __shared__ int warp_tot[NA_TPB / 32];
-    __shared__ int carry;
-    const int ncell = sc->header[0] * sc->header[1] * sc->header[2];
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    if(threadIdx.x == 0) {carry = 0;}
-    __syncthreads();
-    for(int base = 0; base < ncell; base += NA_TPB)
+    __shared__ int header[4];
+    __shared__ double inv_w;
+    if(threadIdx.x == 0)
     {
-        const int c = base + threadIdx.x;
-        const int v = c < ncell ? sc->count[c] : 0;
-        int incl = v;
-        for(int o = 1; o < 32; o <<= 1)
+        int h[4];
+        double w;
+        na_grid(sc, n, cutoff_ratio, box, h, w);
+        for(int k = 0; k < 4; ++k) {header[k] = h[k];}
+        inv_w = w;
+        if(blockIdx.x == 0)
         {
-            const int y = __shfl_up_sync(0xffffffffu, incl, o);
-            if(lane >= o) {incl += y;}
+            for(int k = 0; k < 4; ++k) {sc->header[k] = h[k];}
+            sc->inv_w = w;
         }
-        if(lane == 31) {warp_tot[w] = incl;}
-        __syncthreads();
-        if(w == 0)
-        {
-            const int x = lane < NA_TPB / 32 ? warp_tot[lane] : 0;
-            int xi = x;
-            for(int o = 1; o < 32; o <<= 1)
-            {
-                const int y = __shfl_up_sync(0xffffffffu, xi, o);
-                if(lane >= o) {xi += y;}
-            }
-            if(lane < NA_TPB / 32) {warp_tot[lane] = xi - x;}
-        }
-        __syncthreads();
-        const int excl = carry + warp_tot[w] + incl - v;
-        if(c < ncell) {sc->start[c] = excl;}
-        __syncthreads();
-        if(threadIdx.x == NA_TPB - 1) {carry = excl + v;}
-        __syncthreads();
     }
-    if(threadIdx.x == 0) {sc->start[ncell] = carry;}
+    __syncthreads();
+    const long long i = (long long)blockIdx.x * NA_TPB + threadIdx.x;
+    if(i >= n) {return;}
+    const int c = na_coord(header, inv_w, box, pos[3 * i], 0) + header[0] * (na_coord(header, inv_w, box, pos[3 * i + 1], 1) +
+                  header[1] * na_coord(header, inv_w, box, pos[3 * i + 2], 2));
+    sc->place[i] = (unsigned)c << 16 | (unsigned)atomicAdd(&sc->count[c], 1);
 }
 
-__global__ void k_na_scatter(NaScratch* sc, long long n, const double* pos, NaBox box)
+// exclusive scan of the cell counts, one block per NA_SCAN cells: a block adds up
+// the counts before its own cells itself (at most 256 KB from L2), so the blocks
+// need not wait for one another
+__global__ void __launch_bounds__(NA_SCAN) k_na_scan(NaScratch* sc)
+{
+    __shared__ int tot[32];
+    __shared__ int base;
+    const int ncell = sc->header[0] * sc->header[1] * sc->header[2];
+    const int first = blockIdx.x * NA_SCAN;
+    if(first >= ncell) {return;}
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    int before = 0;
+    for(int c = threadIdx.x; c < first; c += NA_SCAN) {before += sc->count[c];}
+    before = __reduce_add_sync(0xffffffffu, before);
+    const int c = first + threadIdx.x;
+    const int v = c < ncell ? sc->count[c] : 0;
+    int incl = v;
+#pragma unroll
+    for(int o = 1; o < 32; o <<= 1)
+    {
+        const int y = __shfl_up_sync(0xffffffffu, incl, o);
+        if(lane >= o) {incl += y;}
+    }
+    if(threadIdx.x == 0) {base = 0;}
+    if(lane == 31) {tot[w] = incl;}
+    __syncthreads();
+    if(lane == 0 && before) {atomicAdd(&base, before);}
+    __syncthreads();
+    int run = base;
+    for(int k = 0; k < w; ++k) {run += tot[k];}
+    if(c < ncell) {sc->start[c] = run + incl - v;}
+    if(c == ncell - 1) {sc->start[ncell] = run + incl;}
+}
+
+__global__ void __launch_bounds__(NA_TPB) k_na_scatter(NaScratch* sc, long long n)
 {
     const long long i = (long long)blockIdx.x * NA_TPB + threadIdx.x;
     if(i >= n) {return;}
-    const int c = na_cell(sc, na_coord(sc, box, pos[3 * i], 0), na_coord(sc, box, pos[3 * i + 1], 1),
-                          na_coord(sc, box, pos[3 * i + 2], 2));
-    sc->order[sc->start[c] + atomicAdd(&sc->fill[c], 1)] = (int)i;
+    const unsigned p = sc->place[i];
+    sc->order[sc->start[p >> 16] + (int)(p & 0xffffu)] = (int)i;
 }
 
-__global__ void k_na_force(const NaScratch* sc, long long n, const double* pos, const double* radius,
+// Forces, NA_LANES lanes per particle, particles in cell order (neighbouring
+// groups read the same partners).  The 27 cells around a particle are nine rows
+// along x, each one range of the cell order or two where it wraps; the lanes
+// look the at most 18 ranges up together and then walk their concatenation, so
+// a particle's candidates (41 in the bead fluid) are a few loads deep instead of
+// one serial chain through 27 cells.
+constexpr int NA_RANGES = 18;
+__global__ void __launch_bounds__(NA_TPB) k_na_force(const NaScratch* sc, long long n, const double* pos, const double* radius,
                            double eps, double cutoff_ratio, NaBox box, double* force, double* energy)
 {
-    const long long i = (long long)blockIdx.x * NA_TPB + threadIdx.x;
-    double e = 0.0;
-    if(i < n)
+    constexpr int GROUPS = NA_TPB / NA_LANES;
+    __shared__ int s_begin[GROUPS][NA_RANGES];
+    __shared__ int s_excl[GROUPS][NA_RANGES + 1];
+    const unsigned full = 0xffffffffu;
+    const int grp = threadIdx.x / NA_LANES, gl = threadIdx.x % NA_LANES;
+    int* const begin = s_begin[grp];
+    int* const excl = s_excl[grp];
+    const long long slot = (long long)blockIdx.x * GROUPS + grp;
+    const bool valid = slot < n;
+    double e = 0.0, fx = 0.0, fy = 0.0, fz = 0.0;
+    int i = 0;
+    double xi = 0.0, yi = 0.0, zi = 0.0, ri = 0.0;
+    if(valid)
     {
-        const double xi = pos[3 * i], yi = pos[3 * i + 1], zi = pos[3 * i + 2], ri = radius[i];
+        i = sc->order[slot];
+        xi = pos[3 * i]; yi = pos[3 * i + 1]; zi = pos[3 * i + 2]; ri = radius[i];
+        const int cell = (int)(sc->place[i] >> 16);
+        const int nx = sc->header[0], ny = sc->header[1], nz = sc->header[2];
+        const int cx = cell % nx, cy = cell / nx % ny, cz = cell / (nx * ny);
+        for(int j = gl; j < 9; j += NA_LANES)
+        {
+            const int y = (cy + j % 3 - 1 + ny) % ny, z = (cz + j / 3 - 1 + nz) % nz;
+            const int row = nx * (y + ny * z);
+            int lo = cx - 1, hi = cx + 1, hi1 = -1;      // the second range is [0, hi1]
+            if(lo < 0)        {lo = hi = nx - 1; hi1 = cx + 1;}
+            else if(hi >= nx) {hi = nx - 1; hi1 = 0;}
+            begin[2 * j] = sc->start[row + lo];
+            excl[2 * j] = sc->start[row + hi + 1] - begin[2 * j];
+            begin[2 * j + 1] = sc->start[row];
+            excl[2 * j + 1] = sc->start[row + hi1 + 1] - begin[2 * j + 1];
+        }
+    }
+    __syncwarp();
+    if(valid && gl == 0)
+    {
+        int run = 0;
+        for(int k = 0; k < NA_RANGES; ++k)
+        {
+            const int c = excl[k];
+            excl[k] = run;
+            run += c;
+        }
+        excl[NA_RANGES] = run;
+    }
+    __syncwarp();
+    if(valid)
+    {
         const double crsq = cutoff_ratio * cutoff_ratio;
         const double coef_at_cutoff = pow(1.0 / cutoff_ratio, 12);   // ExcludedVolumePotential.hpp:44-48
         const double eps12 = eps * 12;
-        const int dx_ = sc->header[0], dy_ = sc->header[1], dz_ = sc->header[2];
-        const int cx = na_coord(sc, box, xi, 0), cy = na_coord(sc, box, yi, 1), cz = na_coord(sc, box, zi, 2);
-        double fx = 0.0, fy = 0.0, fz = 0.0;
-        for(int oz = -1; oz <= 1; ++oz)
-        for(int oy = -1; oy <= 1; ++oy)
-        for(int ox = -1; ox <= 1; ++ox)
+        const int total = excl[NA_RANGES];
+        int at = 0;
+        auto candidate = [&](int k) {
+            if(k >= total) {return i;}               // none: the particle itself, which is dropped
+            while(at < NA_RANGES - 1 && excl[at + 1] <= k) {++at;}
+            return sc->order[begin[at] + (k - excl[at])];
+        };
+        // the next candidate's coordinates are requested before the current pair is evaluated
+        int j = candidate(gl);
+        double xj = pos[3 * j], yj = pos[3 * j + 1], zj = pos[3 * j + 2], rj = radius[j];
+        for(int k = gl; k < total; k += NA_LANES)
         {
-            const int x = (cx + ox + dx_) % dx_, y = (cy + oy + dy_) % dy_, z = (cz + oz + dz_) % dz_;
-            const int c = na_cell(sc, x, y, z);
-            for(int m = sc->start[c]; m < sc->start[c + 1]; ++m)
+            const int jn = candidate(k + NA_LANES);
+            const double xn = pos[3 * jn], yn = pos[3 * jn + 1], zn = pos[3 * jn + 2], rn = radius[jn];
+            if(j != i)
             {
-                const int j = sc->order[m];
-                if(j == i) {continue;}
-                double ddx = pos[3 * j] - xi, ddy = pos[3 * j + 1] - yi, ddz = pos[3 * j + 2] - zi;
+                double ddx = xj - xi, ddy = yj - yi, ddz = zj - zi;
                 if(box.periodic)
                 {
                     ddx = min_image(ddx, box.halfw[0], box.width[0]);
@@ -210,20 +279,32 @@ __global__ void k_na_force(const NaScratch* sc, long long n, const double* pos, 
                     ddz = min_image(ddz, box.halfw[2], box.width[2]);
                 }
                 const double l_sq = ddx * ddx + ddy * ddy + ddz * ddz;
-                const double sigma = ri + radius[j];
+                const double sigma = ri + rj;
                 const double sigma_sq = sigma * sigma;
-                if(sigma_sq * crsq < l_sq) {continue;}
-                const double rcp = 1.0 / l_sq;
-                const double s2 = sigma_sq * rcp;
-                const double s6 = s2 * s2 * s2;
-                const double cf = -eps12 * s6 * s6 * rcp;
-                fx += ddx * cf; fy += ddy * cf; fz += ddz * cf;
-                if(i < j) {e += eps * (s6 * s6 - coef_at_cutoff);}
+                if(!(sigma_sq * crsq < l_sq))
+                {
+                    const double rcp = 1.0 / l_sq;
+                    const double s2 = sigma_sq * rcp;
+                    const double s6 = s2 * s2 * s2;
+                    const double cf = -eps12 * s6 * s6 * rcp;
+                    fx += ddx * cf; fy += ddy * cf; fz += ddz * cf;
+                    if(i < j) {e += eps * (s6 * s6 - coef_at_cutoff);}
+                }
             }
+            j = jn;
+            xj = xn; yj = yn; zj = zn; rj = rn;
         }
-        force[3 * i] = fx; force[3 * i + 1] = fy; force[3 * i + 2] = fz;
     }
-    for(int o = 16; o > 0; o >>= 1) {e += __shfl_xor_sync(0xffffffffu, e, o);}
+#pragma unroll
+    for(int o = NA_LANES / 2; o > 0; o >>= 1)
+    {
+        fx += __shfl_xor_sync(full, fx, o);
+        fy += __shfl_xor_sync(full, fy, o);
+        fz += __shfl_xor_sync(full, fz, o);
+    }
+    if(valid && gl == 0) {force[3 * i] = fx; force[3 * i + 1] = fy; force[3 * i + 2] = fz;}
+#pragma unroll
+    for(int o = 16; o > 0; o >>= 1) {e += __shfl_xor_sync(full, e, o);}
     if((threadIdx.x & 31) == 0 && e != 0.0) {atomicAdd(energy, e);}
 }
 
@@ -331,10 +412,11 @@ extern "C" MJG_API int mjg_exv_force_noalloc(int64_t n, int boundary, const doub
     }
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     const unsigned nb = (unsigned)((n + NA_TPB - 1) / NA_TPB);
-    k_na_setup  <<<1, NA_TPB, 0, s>>>(sc, n, radius, cutoff_ratio, box, energy);
-    k_na_bin    <<<nb, NA_TPB, 0, s>>>(sc, n, pos, box);
-    k_na_scan   <<<1, NA_TPB, 0, s>>>(sc);
-    k_na_scatter<<<nb, NA_TPB, 0, s>>>(sc, n, pos, box);
-    k_na_force  <<<nb, NA_TPB, 0, s>>>(sc, n, pos, radius, epsilon, cutoff_ratio, box, force, energy);
+    const unsigned nf = (unsigned)((n * NA_LANES + NA_TPB - 1) / NA_TPB);
+    k_na_radius <<<NA_BLOCKS, NA_TPB, 0, s>>>(sc, n, radius, energy);
+    k_na_bin    <<<nb, NA_TPB, 0, s>>>(sc, n, pos, cutoff_ratio, box);
+    k_na_scan   <<<NA_MAX_CELLS / NA_SCAN, NA_SCAN, 0, s>>>(sc);
+    k_na_scatter<<<nb, NA_TPB, 0, s>>>(sc, n);
+    k_na_force  <<<nf, NA_TPB, 0, s>>>(sc, n, pos, radius, epsilon, cutoff_ratio, box, force, energy);
     return cudaGetLastError() == cudaSuccess ? MJG_OK : MJG_ECUDA;
 }
