@@ -99,6 +99,16 @@ struct HostLocal {
     std::vector<int32_t> n;
     int64_t m() const {return (int64_t)k.size();}
 };
+struct LocalRecord {
+    int idx[4];                  // particles, -1 past the last
+    int term[3];                 // bond, angle, dihedral of the system, -1: none
+};
+inline int smallest_particle(const LocalRecord& r)
+{
+    int m = std::min(r.idx[0], r.idx[1]);
+    for(int k = 2; k < 4; ++k) {if(r.idx[k] >= 0) {m = std::min(m, r.idx[k]);}}
+    return m;
+}
 struct HostSystem {
     bool alive = true;
     bool resident = false;       // part of the current arena
@@ -128,6 +138,7 @@ struct HostSystem {
     std::vector<int32_t> mol_local;
     std::vector<long long> ex_start_local[NGLOBAL];   // n + 1 entries
     std::vector<int> ex_idx_local[NGLOBAL];
+    std::vector<LocalRecord> records;                 // bonded terms joined for the step's forces
 };
 
 struct TermDev {
@@ -185,7 +196,7 @@ struct mjg_context {
     mjg::DevBuf l_bond_idx, l_bond_k, l_bond_v0, l_bond_sys;
     mjg::DevBuf l_angle_idx, l_angle_k, l_angle_v0, l_angle_sys;
     mjg::DevBuf l_dihd_idx, l_dihd_k, l_dihd_n, l_dihd_v0, l_dihd_sys;
-    mjg::DevBuf l_win_bond, l_win_angle, l_win_dihd, l_bond_kv, l_angle_kv, l_dihd_p;
+    mjg::DevBuf l_win_bond, l_win_angle, l_win_dihd, l_rec, l_bond_kv, l_angle_kv, l_dihd_p;
     mjg::Arena arena{};
     mjg::LocalArrays local{};
     std::vector<mjg::SysDev> h_sys;
@@ -213,7 +224,7 @@ int64_t device_bytes(const mjg_context* c)
                             &c->l_bond_sys, &c->l_angle_idx, &c->l_angle_k, &c->l_angle_v0,
                             &c->l_angle_sys, &c->l_dihd_idx, &c->l_dihd_k, &c->l_dihd_n,
                             &c->l_dihd_v0, &c->l_dihd_sys, &c->l_win_bond, &c->l_win_angle,
-                            &c->l_win_dihd, &c->l_bond_kv, &c->l_angle_kv, &c->l_dihd_p};
+                            &c->l_win_dihd, &c->l_rec, &c->l_bond_kv, &c->l_angle_kv, &c->l_dihd_p};
     for(auto* x : bufs) {b += (int64_t)x->cap;}
     for(const auto& t : c->term)
     {
@@ -611,11 +622,73 @@ TopologyGraph topology_of(const HostSystem& s, std::map<std::string, int>& kinds
     return topo;
 }
 
+// Joins the system's bonded terms into records (local_terms.cuh): a dihedral
+// takes the angle over its first three particles and the bond over its first
+// two, an angle left over the bond over its first two, each term once; the
+// records are put in order of their smallest particle.
+void join_terms(HostSystem& s)
+{
+    // terms by their first particle: the last one, then links to earlier ones
+    auto chain = [&](const HostLocal& L, int arity, std::vector<int>& head, std::vector<int>& next) {
+        head.assign((size_t)s.n, -1);
+        next.assign((size_t)L.m(), -1);
+        for(int64_t t = L.m() - 1; t >= 0; --t)
+        {
+            int& h = head[(size_t)L.idx[arity * t]];
+            next[(size_t)t] = h;
+            h = (int)t;
+        }
+    };
+    std::vector<int> bh, bn, ah, an;
+    chain(s.bond, 2, bh, bn);
+    chain(s.angle, 3, ah, an);
+    std::vector<char> bond_used((size_t)s.bond.m(), 0), angle_used((size_t)s.angle.m(), 0);
+    auto take_bond = [&](const int64_t* q) {
+        for(int t = bh[(size_t)q[0]]; t >= 0; t = bn[(size_t)t])
+        {
+            if(!bond_used[(size_t)t] && s.bond.idx[2 * (size_t)t + 1] == q[1]) {bond_used[(size_t)t] = 1; return t;}
+        }
+        return -1;
+    };
+    auto take_angle = [&](const int64_t* q) {
+        for(int t = ah[(size_t)q[0]]; t >= 0; t = an[(size_t)t])
+        {
+            const int64_t* w = &s.angle.idx[3 * (size_t)t];
+            if(!angle_used[(size_t)t] && w[1] == q[1] && w[2] == q[2]) {angle_used[(size_t)t] = 1; return t;}
+        }
+        return -1;
+    };
+    std::vector<LocalRecord>& R = s.records;
+    R.clear();
+    R.reserve((size_t)std::max(s.bond.m(), std::max(s.angle.m(), s.dihd.m())));
+    for(int64_t t = 0; t < s.dihd.m(); ++t)
+    {
+        const int64_t* q = &s.dihd.idx[4 * t];
+        R.push_back({{(int)q[0], (int)q[1], (int)q[2], (int)q[3]}, {take_bond(q), take_angle(q), (int)t}});
+    }
+    for(int64_t t = 0; t < s.angle.m(); ++t)
+    {
+        if(angle_used[(size_t)t]) {continue;}
+        const int64_t* q = &s.angle.idx[3 * t];
+        R.push_back({{(int)q[0], (int)q[1], (int)q[2], -1}, {take_bond(q), (int)t, -1}});
+    }
+    for(int64_t t = 0; t < s.bond.m(); ++t)
+    {
+        if(bond_used[(size_t)t]) {continue;}
+        const int64_t* q = &s.bond.idx[2 * t];
+        R.push_back({{(int)q[0], (int)q[1], -1, -1}, {(int)t, -1, -1}});
+    }
+    std::stable_sort(R.begin(), R.end(), [](const LocalRecord& x, const LocalRecord& y) {
+        return smallest_particle(x) < smallest_particle(y);
+    });
+}
+
 // the per-system data that depends on topology only (molecules, exclusion
 // lists), computed once in the edge order the reference's local force field
 // writes the topology, after which the local terms are put in order of their
-// smallest particle (the order the bonded kernel walks them in)
-void derive(HostSystem& s)
+// smallest particle (the order the bonded kernel walks them in) and, for the
+// mixed form, joined into records
+void derive(HostSystem& s, bool join)
 {
     if(s.derived) {return;}
     std::map<std::string, int> kinds;
@@ -665,6 +738,7 @@ void derive(HostSystem& s)
     order(s.bond, 2);
     order(s.angle, 3);
     order(s.dihd, 4);
+    if(join) {join_terms(s);}
     s.derived = true;
 }
 
@@ -869,7 +943,7 @@ void commit(mjg_context* c)
         ids.push_back(i);
     }
     const int nsys = (int)ids.size();
-    parallel_for(nsys, [&](int64_t k) {derive(c->sys[ids[k]]);});
+    parallel_for(nsys, [&](int64_t k) {derive(c->sys[ids[k]], c->precision == P_MIXED);});
     tm.mark("derive");
 
     // ---- offsets (serial, per system)
@@ -878,7 +952,7 @@ void commit(mjg_context* c)
     std::vector<SysDev> hs(nsys);
     parallel_for(nsys, [&](int64_t k) {make_sysdev(c->sys[ids[k]], hs[k]);});
     std::vector<long long> mol_base(nsys + 1, 0), ex_off[NGLOBAL], b_off(nsys + 1, 0), a_off(nsys + 1, 0),
-                           d_off(nsys + 1, 0);
+                           d_off(nsys + 1, 0), r_off(nsys + 1, 0);
     long long np_tot[NGLOBAL] = {0, 0, 0}, ncell[NGLOBAL] = {0, 0, 0};
     long long part_chunk_cap[NGLOBAL] = {0, 0, 0}, cell_chunk_cap[NGLOBAL] = {0, 0, 0};
     for(int g = 0; g < NGLOBAL; ++g) {ex_off[g].assign(nsys + 1, 0);}
@@ -905,12 +979,13 @@ void commit(mjg_context* c)
         b_off[k + 1] = b_off[k] + s.bond.m();
         a_off[k + 1] = a_off[k] + s.angle.m();
         d_off[k + 1] = d_off[k] + s.dihd.m();
+        r_off[k + 1] = r_off[k] + (long long)s.records.size();
     }
     for(int g = 0; g < NGLOBAL; ++g)
     {
         if(np_tot[g] > INT32_MAX || ncell[g] > INT32_MAX) {throw Error(MJG_EINVAL, "arena too large");}
     }
-    const long long nb = b_off[nsys], na = a_off[nsys], nd = d_off[nsys];
+    const long long nb = b_off[nsys], na = a_off[nsys], nd = d_off[nsys], nr = r_off[nsys];
     const int nwin = (int)((n_tot + 255) / 256);
 
     // ---- layout of the page-locked packing buffer
@@ -935,6 +1010,8 @@ void commit(mjg_context* c)
                c_dsys = cv.add<int>(nd), c_dn = cv.add<int>(nd), c_dp = cv.add<float4>(nd);
     const auto c_wb = cv.add<long long>(nwin + 1), c_wa = cv.add<long long>(nwin + 1),
                c_wd = cv.add<long long>(nwin + 1);
+    // the records in one device buffer: particles, terms, windows
+    const auto c_rec = cv.add<char>(32 * (size_t)nr + sizeof(long long) * (nwin + 1));
     if(cv.total > c->h_pack_bytes)
     {
         if(c->h_pack) {cudaFreeHost(c->h_pack); c->h_pack = nullptr; c->h_pack_bytes = 0;}
@@ -952,6 +1029,7 @@ void commit(mjg_context* c)
     int* a_sys = (int*)at(c_asys); float2* a_kv = (float2*)at(c_akv);
     int* d_idx = (int*)at(c_didx); double* d_k = (double*)at(c_dk); double* d_v0 = (double*)at(c_dv0);
     int* d_sys = (int*)at(c_dsys); int* d_n = (int*)at(c_dn); float4* d_p = (float4*)at(c_dp);
+    int4* r_idx = (int4*)at(c_rec); int4* r_term = r_idx + nr;
     tm.mark("layout");
 
     // ---- fill (parallel over systems)
@@ -1038,6 +1116,16 @@ void commit(mjg_context* c)
                 p1[x] = H.p1.empty() ? 0.0 : H.p1[q];
             }
         }
+        for(size_t t = 0; t < s.records.size(); ++t)
+        {
+            const LocalRecord& q = s.records[t];
+            const long long x = r_off[k] + (long long)t;
+            auto particle = [&](int i) {return i < 0 ? -1 : (int)(off + i);};
+            r_idx[x] = make_int4(particle(q.idx[0]), particle(q.idx[1]), particle(q.idx[2]), particle(q.idx[3]));
+            r_term[x] = make_int4((int)k, q.term[0] < 0 ? -1 : (int)(b_off[k] + q.term[0]),
+                                  q.term[1] < 0 ? -1 : (int)(a_off[k] + q.term[1]),
+                                  q.term[2] < 0 ? -1 : (int)(d_off[k] + q.term[2]));
+        }
         for(int64_t t = 0; t < s.bond.m(); ++t)
         {
             const long long x = b_off[k] + t;
@@ -1070,13 +1158,14 @@ void commit(mjg_context* c)
     // local terms: every system keeps its terms ordered by their smallest
     // particle and systems are packed in order, so the arena's terms are in
     // order too; CSR of terms over 256-particle windows
+    // (negative indices: no particle)
     auto windows = [&](const int* idx, int arity, long long m, long long* win) {
         std::fill(win, win + nwin + 1, 0LL);
         int prev = 0;
         for(long long t = 0; t < m; ++t)
         {
             int mn = idx[arity * t];
-            for(int x = 1; x < arity; ++x) {mn = std::min(mn, idx[arity * t + x]);}
+            for(int x = 1; x < arity; ++x) {if(idx[arity * t + x] >= 0) {mn = std::min(mn, idx[arity * t + x]);}}
             if(mn < prev) {throw Error(MJG_ESTATE, "local terms out of order");}
             prev = mn;
             win[mn / 256 + 1] += 1;
@@ -1086,6 +1175,7 @@ void commit(mjg_context* c)
     windows(b_idx, 2, nb, (long long*)at(c_wb));
     windows(a_idx, 3, na, (long long*)at(c_wa));
     windows(d_idx, 4, nd, (long long*)at(c_wd));
+    windows(reinterpret_cast<const int*>(r_idx), 4, nr, reinterpret_cast<long long*>(r_term + nr));
     tm.mark("fill");
 
     // ---- device upload (buffers keep their capacity across commits)
@@ -1277,6 +1367,7 @@ void commit(mjg_context* c)
     LocalArrays& l = c->local;
     l = LocalArrays{};
     put(c->l_bond_kv, c_bkv); put(c->l_angle_kv, c_akv); put(c->l_dihd_p, c_dp);
+    put(c->l_rec, c_rec);
     put(c->l_win_bond, c_wb); put(c->l_win_angle, c_wa); put(c->l_win_dihd, c_wd);
     put(c->l_bond_idx, c_bidx);  put(c->l_bond_k, c_bk);
     put(c->l_bond_v0, c_bv0);    put(c->l_bond_sys, c_bsys);
@@ -1294,6 +1385,10 @@ void commit(mjg_context* c)
     l.dihd_n = c->l_dihd_n.as<int>();       l.dihd_v0 = c->l_dihd_v0.as<double>();
     l.dihd_sys = c->l_dihd_sys.as<int>();
     l.nwin = nwin;
+    l.nrec = nr;
+    l.rec_idx = c->l_rec.as<int4>();
+    l.rec_term = l.rec_idx + nr;
+    l.win_rec = reinterpret_cast<const long long*>(l.rec_term + nr);
     l.bond_kv = c->l_bond_kv.as<float2>();
     l.angle_kv = c->l_angle_kv.as<float2>();
     l.dihd_p = c->l_dihd_p.as<float4>();

@@ -129,6 +129,14 @@ struct LocalArrays {
     const float2* bond_kv;
     const float2* angle_kv;
     const float4* dihd_p;
+    // the same terms joined into records for the step's forces (see
+    // local_terms.cuh), sorted by their smallest particle: particles {i0, i1,
+    // i2, i3} (-1 past the last one) and {system, bond, angle, dihedral} (term
+    // indices, -1 where the record has none)
+    long long nrec;
+    const int4* rec_idx;
+    const int4* rec_term;
+    const long long* win_rec;
     // terms sorted by their smallest particle index; window w of 256 particles
     // owns terms win_x[w] .. win_x[w + 1]
     int nwin;

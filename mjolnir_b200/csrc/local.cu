@@ -18,6 +18,9 @@ namespace mjg {
 namespace {
 
 constexpr int TPB = 256;
+// blocks per SM of the record kernel: 64 registers each; 3 (80 registers) and 5
+// (48, spilling) were slower (100 steps of 256 melts 38.3 ms; 39.4 and 38.8)
+constexpr int LOCAL_BLOCKS = 4;
 
 // One block per window of SEG particles: every bond, angle and dihedral whose
 // smallest particle index falls in the window (terms are sorted by it at
@@ -46,7 +49,7 @@ __global__ void __launch_bounds__(TPB, PREC == P_MIXED ? 5 : 3) k_local(Arena a,
         {
             const long long b = base + threadIdx.x;
             if(PREC == P_FP64) {do_bond<PREC, NF, NE>(a, l, b, b < b1 && !(a.any_frozen && a.sys[l.bond_sys[b]].frozen), W);}
-            else               {do_bond_f32<PREC, NF, NE>(a, l, b, b < b1 && !(a.any_frozen && a.sys[l.bond_sys[b]].frozen), W);}
+            else               {if(b < b1 && !(a.any_frozen && a.sys[l.bond_sys[b]].frozen)) {do_bond_f32(a, l, b, W);}}
         }
     }
     if(mask & 2)
@@ -56,7 +59,7 @@ __global__ void __launch_bounds__(TPB, PREC == P_MIXED ? 5 : 3) k_local(Arena a,
         {
             const long long b = base + threadIdx.x;
             if(PREC == P_FP64) {do_angle<PREC, NF, NE>(a, l, b, b < b1 && !(a.any_frozen && a.sys[l.angle_sys[b]].frozen), W);}
-            else               {do_angle_f32<PREC, NF, NE>(a, l, b, b < b1 && !(a.any_frozen && a.sys[l.angle_sys[b]].frozen), W);}
+            else               {if(b < b1 && !(a.any_frozen && a.sys[l.angle_sys[b]].frozen)) {do_angle_f32(a, l, b, W);}}
         }
     }
     if(mask & 4)
@@ -66,7 +69,7 @@ __global__ void __launch_bounds__(TPB, PREC == P_MIXED ? 5 : 3) k_local(Arena a,
         {
             const long long b = base + threadIdx.x;
             if(PREC == P_FP64) {do_dihedral<PREC, NF, NE>(a, l, b, b < b1 && !(a.any_frozen && a.sys[l.dihd_sys[b]].frozen), W);}
-            else               {do_dihedral_f32<PREC, NF, NE>(a, l, b, b < b1 && !(a.any_frozen && a.sys[l.dihd_sys[b]].frozen), W);}
+            else               {if(b < b1 && !(a.any_frozen && a.sys[l.dihd_sys[b]].frozen)) {do_dihedral_f32(a, l, b, W);}}
         }
     }
     if(NF)
@@ -74,6 +77,55 @@ __global__ void __launch_bounds__(TPB, PREC == P_MIXED ? 5 : 3) k_local(Arena a,
         __syncthreads();
         W.flush(a.force, a.n);
     }
+}
+
+// The mixed form's bonded forces of a step: one block per window of SEG
+// particles, a thread per record (local_terms.cuh), summed in the window as
+// above.  The terms that need the FP64 formulas are put aside in shared memory and
+// done by the block's threads side by side: a few in a hundred of them (a chain
+// whose angles relax from a random walk) are enough to reach every warp, and each
+// warp would then wait for the long FP64 evaluation of one or two lanes (256 melts
+// from their first frame: 127 us with the FP64 formulas in line, 89 put aside; 114
+// for the separate terms).
+struct DeferringWindow : Window<P_MIXED> {
+    static constexpr bool DEFER = true;
+    int* count;          // [2] angles, dihedrals put aside
+    int* queue;          // [2][TPB]
+    __device__ __forceinline__ void defer_angle(int t)    {queue[atomicAdd(&count[0], 1)] = t;}
+    __device__ __forceinline__ void defer_dihedral(int t) {queue[TPB + atomicAdd(&count[1], 1)] = t;}
+};
+
+__global__ void __launch_bounds__(TPB, LOCAL_BLOCKS) k_local_records(Arena a, LocalArrays l)
+{
+    __shared__ unsigned win[Window<P_MIXED>::SIZE];
+    __shared__ int queue[2 * TPB];
+    __shared__ int count[2];
+    const int w = blockIdx.x;
+    DeferringWindow W;
+    W.w = win; W.base = w * SEG; W.count = count; W.queue = queue;
+    for(int k = threadIdx.x; k < Window<P_MIXED>::SIZE; k += TPB) {win[k] = 0;}
+    if(threadIdx.x < 2) {count[threadIdx.x] = 0;}
+    __syncthreads();
+    const long long end = l.win_rec[w + 1];
+    for(long long first = l.win_rec[w]; first < end; first += TPB)
+    {
+        const long long r = first + threadIdx.x;
+        if(r < end) {do_record(a, l, r, W);}
+        __syncthreads();
+        // angles by the first half of the block, dihedrals by the second
+        const int half = threadIdx.x / (TPB / 2);
+        const int n = count[half];
+        Window<P_MIXED>& V = W;
+        for(int k = threadIdx.x % (TPB / 2); k < n; k += TPB / 2)
+        {
+            if(half == 0) {angle_fp64<P_MIXED, true, false>(a, l, queue[k], V);}
+            else          {dihedral_fp64<P_MIXED, true, false>(a, l, queue[TPB + k], V);}
+        }
+        __syncthreads();
+        if(threadIdx.x < 2) {count[threadIdx.x] = 0;}
+        __syncthreads();
+    }
+    W.flush(a.force, a.n);
 }
 
 template<int PREC, bool NF, bool NE>
@@ -89,6 +141,13 @@ void run_all(const Arena& a, const LocalArrays& l, int mask, cudaStream_t s)
 void launch_local(const Arena& a, const LocalArrays& l, int mask, bool nf, bool ne,
                   int /*calc_energy_form*/, cudaStream_t s)
 {
+    if(a.precision == P_MIXED && mask == 7 && nf && !ne)
+    {
+        if(l.nwin == 0 || l.nrec == 0) {return;}
+        k_local_records<<<l.nwin, TPB, 0, s>>>(a, l);
+        note_launches(1);
+        return;
+    }
     if(a.precision == P_FP64)
     {
         if(nf && ne) {run_all<P_FP64, true, true>(a, l, mask, s);}

@@ -101,9 +101,14 @@ struct Barrier {
 // block-wide window of the bonded launch would only lengthen the chain.
 template<int PREC>
 struct DirectAdd {
+    static constexpr bool DEFER = false;   // mixed form
     __device__ __forceinline__ void add(void* force, int i, double fx, double fy, double fz)
     {
         Window<PREC>::global_add(force, i, fx, fy, fz);
+    }
+    __device__ __forceinline__ void add_fx(void* force, int i, long long x, long long y, long long z)
+    {
+        Window<PREC>::global_add_fx(force, i, x, y, z);
     }
 };
 
@@ -329,33 +334,39 @@ __device__ __forceinline__ void pair_item(const Arena& a, const TermArrays& t, i
     if(ovf) {atomicOr(&a.sys[head.sys].status, ST_FIXED_OVERFLOW);}
 }
 
+__host__ __device__ inline int warps_of(long long n) {return (int)((n + 31) / 32);}
+
+// Warp item e of the bonded terms: records in the mixed form; in the plain form,
+// whose formulas are long enough that one thread's three terms in a row would
+// set the phase's time, dihedrals, angles and bonds by themselves.
 template<int PREC>
-__device__ __forceinline__ void local_item(const Arena& a, const LocalArrays& l, int kind, int e)
+__device__ __forceinline__ void local_item(const Arena& a, const LocalArrays& l, int e)
 {
-    const long long b = (long long)e * 32 + (threadIdx.x & 31);
+    const int lane = threadIdx.x & 31;
     DirectAdd<PREC> W;
-    if(kind == 0)
+    if constexpr(PREC == P_MIXED)
     {
-        if(b >= l.nbond || (a.any_frozen && a.sys[l.bond_sys[b]].frozen)) {return;}
-        if(PREC == P_FP64) {do_bond<PREC, true, false>(a, l, b, true, W);}
-        else               {do_bond_f32<PREC, true, false>(a, l, b, true, W);}
-    }
-    else if(kind == 1)
-    {
-        if(b >= l.nangle || (a.any_frozen && a.sys[l.angle_sys[b]].frozen)) {return;}
-        if(PREC == P_FP64) {do_angle<PREC, true, false>(a, l, b, true, W);}
-        else               {do_angle_f32<PREC, true, false>(a, l, b, true, W);}
+        const long long b = (long long)e * 32 + lane;
+        if(b < l.nrec) {do_record(a, l, b, W);}
     }
     else
     {
-        if(b >= l.ndihd || (a.any_frozen && a.sys[l.dihd_sys[b]].frozen)) {return;}
-        if(PREC == P_FP64) {do_dihedral<PREC, true, false>(a, l, b, true, W);}
-        else               {do_dihedral_f32<PREC, true, false>(a, l, b, true, W);}
+        const int n_di = warps_of(l.ndihd), n_an = warps_of(l.nangle);
+        const int kind = e < n_di ? 2 : (e < n_di + n_an ? 1 : 0);
+        const long long b = (long long)(e - (kind == 2 ? 0 : (kind == 1 ? n_di : n_di + n_an))) * 32 + lane;
+        if(b >= (kind == 2 ? l.ndihd : (kind == 1 ? l.nangle : l.nbond))) {return;}
+        if(a.any_frozen && a.sys[kind == 2 ? l.dihd_sys[b] : (kind == 1 ? l.angle_sys[b] : l.bond_sys[b])].frozen) {return;}
+        if(kind == 2)      {dihedral_fp64<PREC, true, false>(a, l, b, W);}
+        else if(kind == 1) {angle_fp64<PREC, true, false>(a, l, b, W);}
+        else               {do_bond<PREC, true, false>(a, l, b, true, W);}
     }
+}
+__host__ __device__ inline int local_items(int precision, const LocalArrays& l)
+{
+    return precision == P_MIXED ? warps_of(l.nrec) : warps_of(l.ndihd) + warps_of(l.nangle) + warps_of(l.nbond);
 }
 
 __host__ __device__ inline int pair_items(const TermArrays& t) {return t.on ? (int)((t.np * t.tpp + 31) / 32) : 0;}
-__host__ __device__ inline int warps_of(long long n) {return (int)((n + 31) / 32);}
 
 // The step's forces, longest items first: the dense DebyeHuckel lists, the
 // other pair terms, then the bonded terms.
@@ -363,8 +374,7 @@ template<int PREC>
 __device__ __forceinline__ void forces(const Arena& a, const RunArgs& r, const Grid& G)
 {
     const int n_dh = pair_items(r.t[G_DH]), n_lj = pair_items(r.t[G_LJ]), n_ex = pair_items(r.t[G_EXV]);
-    const int n_di = warps_of(r.l.ndihd), n_an = warps_of(r.l.nangle), n_bo = warps_of(r.l.nbond);
-    const int total = n_dh + n_lj + n_ex + n_di + n_an + n_bo;
+    const int total = n_dh + n_lj + n_ex + local_items(PREC, r.l);
     for(int e = G.warp; e < total; e += G.nwarp)
     {
         int k = e;
@@ -373,11 +383,7 @@ __device__ __forceinline__ void forces(const Arena& a, const RunArgs& r, const G
         if(k < n_lj) {pair_item<PREC, G_LJ>(a, r.t[G_LJ], k); continue;}
         k -= n_lj;
         if(k < n_ex) {pair_item<PREC, G_EXV>(a, r.t[G_EXV], k); continue;}
-        k -= n_ex;
-        if(k < n_di) {local_item<PREC>(a, r.l, 2, k); continue;}
-        k -= n_di;
-        if(k < n_an) {local_item<PREC>(a, r.l, 1, k); continue;}
-        local_item<PREC>(a, r.l, 0, k - n_an);
+        local_item<PREC>(a, r.l, k - n_ex);
     }
 }
 
@@ -511,7 +517,7 @@ cudaError_t launch_run(RunArgs r, int sms, cudaStream_t s)
     // blocks: a warp per item of the force phase, at most one block per SM
     int items = 0;
     for(int g = 0; g < NGLOBAL; ++g) {items += pair_items(r.t[g]);}
-    items += warps_of(r.l.nbond) + warps_of(r.l.nangle) + warps_of(r.l.ndihd);
+    items += local_items(r.a.precision, r.l);
     items = std::max(items, warps_of(r.a.n));
     int blocks = std::max(1, std::min(sms, (items + RT / 32 - 1) / (RT / 32)));
     r.cluster = blocks <= RUN_CLUSTER_MAX ? 1 : 0;
