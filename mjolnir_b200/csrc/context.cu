@@ -1530,7 +1530,8 @@ void run_steps(mjg_context* c, int64_t nsteps)
     cudaStream_t st = c->stream;
     for(int attempt = 0; attempt < 8; ++attempt)
     {
-        if(c->rollback)
+        const bool multi = c->graphs && run_fits(c);
+        if(c->rollback && !multi)                   // the multi-step kernel copies the state itself
         {
             CK(cudaMemcpyAsync(c->b_sys.p, c->d_sys.p, c->d_sys.bytes, cudaMemcpyDeviceToDevice, st));
             CK(cudaMemcpyAsync(c->b_pos.p, c->d_pos.p, c->d_pos.bytes, cudaMemcpyDeviceToDevice, st));
@@ -1543,7 +1544,7 @@ void run_steps(mjg_context* c, int64_t nsteps)
         }
         // step 1 of the chunk, then steps 2..n with the previous closing
         // half-kick fused into their first pass, then the last closing kick
-        if(c->graphs && run_fits(c))
+        if(multi)
         {
             RunArgs r{};
             r.a = c->arena;
@@ -1555,6 +1556,12 @@ void run_steps(mjg_context* c, int64_t nsteps)
             {
                 r.nsteps = (int)std::min<int64_t>(RUN_STEPS, nsteps - k);
                 r.kick = k > 0 ? 1 : 0;
+                const bool copy = c->rollback && k == 0;
+                r.b_sys = copy ? c->b_sys.as<SysDev>() : nullptr;
+                r.b_pos = copy ? c->b_pos.as<double4>() : nullptr;
+                r.b_vel = copy ? c->b_vel.as<double4>() : nullptr;
+                r.b_force = copy ? c->b_force.as<longlong4>() : nullptr;
+                r.b_accel = copy ? c->b_accel.as<double4>() : nullptr;
                 r.close = k + r.nsteps == nsteps ? 1 : 0;
                 CK(launch_run(r, c->sms, st));
             }
@@ -1573,7 +1580,7 @@ void run_steps(mjg_context* c, int64_t nsteps)
         {
             for(int64_t k = 0; k < nsteps; ++k) {enqueue_step_body(c, k > 0, false);}
         }
-        if(!(c->graphs && run_fits(c))) {launch_integrate_last(c->arena, st);}
+        if(!multi) {launch_integrate_last(c->arena, st);}
         CK(cudaGetLastError());
         download_sys(c);
         bool overflow = false;

@@ -169,6 +169,12 @@ struct RunArgs {
     LocalArrays l;
     unsigned* barrier;               // arrival word of the grid barrier (zero before its first use)
     unsigned long long* disp2;       // [2 nsys] largest squared displacements, zero between launches
+    // copies of the state before the launch, for a rollback (nullptr: none wanted)
+    SysDev* b_sys;
+    double4* b_pos;
+    double4* b_vel;
+    longlong4* b_force;              // the bits of either form
+    double4* b_accel;
     int nsteps;
     int kick;                        // open with the closing half of the step before this launch
     int close;                       // end with the closing half of the last step

@@ -404,7 +404,12 @@ __global__ void __launch_bounds__(RT, 1) k_run(const __grid_constant__ RunArgs r
     {
         static_assert(sizeof(SysDev) % sizeof(int4) == 0, "copied in 16-byte words");
         const int4* src = reinterpret_cast<const int4*>(r.a.sys);
-        for(int w = threadIdx.x; w < nsys * (int)(sizeof(SysDev) / sizeof(int4)); w += RT) {reinterpret_cast<int4*>(dyn)[w] = src[w];}
+        for(int w = threadIdx.x; w < nsys * (int)(sizeof(SysDev) / sizeof(int4)); w += RT)
+        {
+            const int4 v = src[w];
+            reinterpret_cast<int4*>(dyn)[w] = v;
+            if(blockIdx.x == 0 && r.b_pos) {reinterpret_cast<int4*>(r.b_sys)[w] = v;}
+        }
         for(int w = threadIdx.x; w < nsys * NGLOBAL; w += RT) {(&sh.rebuilds[0][0])[w] = 0;}
     }
     __syncthreads();
@@ -429,6 +434,13 @@ __global__ void __launch_bounds__(RT, 1) k_run(const __grid_constant__ RunArgs r
         {
             const int s = i == i0 ? sys0 : (i < a.n ? a.psys[i] : -1);
             double d2 = 0.0;
+            if(k == 0 && r.b_pos && s >= 0)       // the state before the chunk
+            {
+                r.b_pos[i] = a.pos[i];
+                r.b_vel[i] = a.vel[i];
+                r.b_force[i] = static_cast<const longlong4*>(a.force)[i];
+                if(AUX) {r.b_accel[i] = a.accel[i];}
+            }
             if(s >= 0 && !sys[s].frozen)
             {
                 SysDev& S = sys[s];
