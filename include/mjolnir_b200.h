@@ -70,7 +70,7 @@ MJG_API int  mjg_context_set_graphs(mjg_context* ctx, int enable);
  * and rolled back when it happens (default 1). */
 MJG_API int  mjg_context_set_rollback(mjg_context* ctx, int enable);
 /* Reserves the page-locked host buffers that commits pack into for an
- * arena of up to `particles` particles (about 450 bytes per particle), so
+ * arena of up to `particles` particles (about 490 bytes per particle), so
  * that a server which fills its arena over many commits does not page-lock
  * memory again and again while it serves.  Optional; buffers still grow
  * when a commit needs more. */

@@ -1710,8 +1710,8 @@ int mjg_context_reserve(mjg_context* c, int64_t particles)
     ABI_BEGIN(c)
     if(particles < 0) {throw Error(MJG_EINVAL, "negative particle count");}
     // the commit's packing buffer: state, coefficients, exclusions, pair
-    // participants and bonded terms come to about 400 bytes per particle
-    const size_t pack = (size_t)particles * 400;
+    // participants, bonded terms and their records come to about 440 bytes per particle
+    const size_t pack = (size_t)particles * 440;
     if(pack > c->h_pack_bytes)
     {
         if(c->h_pack) {cudaFreeHost(c->h_pack); c->h_pack = nullptr; c->h_pack_bytes = 0;}
