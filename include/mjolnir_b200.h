@@ -69,6 +69,13 @@ MJG_API int  mjg_context_set_graphs(mjg_context* ctx, int enable);
 /* Options: the per-step work of mjg_step is also checked for list overflow
  * and rolled back when it happens (default 1). */
 MJG_API int  mjg_context_set_rollback(mjg_context* ctx, int enable);
+/* Limit, in clock cycles of an SM, of a wait between the blocks of the
+ * launch that runs many steps of a small arena (0: the default of 2^31, about a
+ * second).  When a wait runs out, the current mjg_step chunk is rolled back and
+ * runs again as separate launches; with rollback disabled mjg_step returns
+ * MJG_ECUDA, the particles may be a step apart, and further steps are refused
+ * until mjg_commit.  Used to test that path. */
+MJG_API int  mjg_context_set_wait_limit(mjg_context* ctx, int64_t cycles);
 /* Reserves the page-locked host buffers that commits pack into for an
  * arena of up to `particles` particles (about 490 bytes per particle), so
  * that a server which fills its arena over many commits does not page-lock

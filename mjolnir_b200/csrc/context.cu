@@ -188,6 +188,8 @@ struct mjg_context {
     mjg::DevBuf d_force_scratch;
     mjg::DevBuf d_run;                      // multi-step kernel: barrier word, displacements
     int sms = 0;                            // SMs of the device
+    int64_t wait_cycles = mjg::RUN_WAIT_CYCLES;   // limit of a wait inside the multi-step kernel
+    bool torn = false;                      // a chunk stopped half-way and could not be rolled back
     double* h_pinned = nullptr;             // page-locked host staging (state, forces)
     size_t h_pinned_bytes = 0;
     void* h_pack = nullptr;                 // page-locked packing buffer of commit
@@ -494,9 +496,10 @@ void rebuild_all(mjg_context* c)
             CK(cudaStreamSynchronize(c->stream));
         }
     }
-    // rebuild_all may have raised ST_LIST_OVERFLOW on the way; clear it
+    // rebuild_all may have raised ST_LIST_OVERFLOW on the way; clear it (and
+    // what a chunk that has been rolled back left)
     download_sys(c);
-    for(auto& s : c->h_sys) {s.status &= ~ST_LIST_OVERFLOW;}
+    for(auto& s : c->h_sys) {s.status &= ~(ST_LIST_OVERFLOW | ST_BARRIER);}
     upload_sys(c);
 }
 
@@ -1398,6 +1401,7 @@ void commit(mjg_context* c)
     tm.mark("upload");
 
     c->committed = true;
+    c->torn = false;
     rebuild_all(c);
     tm.mark("rebuild");
     compute_initial_forces(c);
@@ -1489,11 +1493,6 @@ void check_status(mjg_context* c, bool& overflow)
     // a list overflow is handled (rolled back) before anything else is checked
     for(const auto& d : c->h_sys) {if(d.status & ST_LIST_OVERFLOW) {overflow = true;}}
     if(overflow) {return;}
-    if(!c->h_sys.empty() && (c->h_sys[0].status & ST_BARRIER))
-    {
-        cudaMemsetAsync(c->d_run.p, 0, c->d_run.bytes, c->stream);   // the arrival word stopped half-way
-        throw Error(MJG_ECUDA, "a grid barrier of the multi-step kernel ran out of time");
-    }
     for(size_t k = 0; k < c->h_sys.size(); ++k)
     {
         const int st = c->h_sys[k].status;
@@ -1524,13 +1523,30 @@ bool run_fits(const mjg_context* c)
     return c->arena.n > 0 && c->arena.n <= RUN_MAX_PARTICLES && c->arena.nsys <= RUN_MAX_SYSTEMS;
 }
 
+// After a wait inside the multi-step kernel ran out: the arrival word and the
+// displacements, and the counters of a rebuild that stopped between its phases
+// (every rebuild expects them zero; a count left over would send slots past the
+// term's arrays).
+void clear_stalled(mjg_context* c)
+{
+    CK(cudaMemsetAsync(c->d_run.p, 0, c->d_run.bytes, c->stream));
+    for(auto& T : c->term)
+    {
+        if(!T.t.on) {continue;}
+        CK(cudaMemsetAsync(T.cell_count.p, 0, T.cell_count.bytes, c->stream));
+        CK(cudaMemsetAsync(T.cell_sum.p, 0, T.cell_sum.bytes, c->stream));
+    }
+}
+
 void run_steps(mjg_context* c, int64_t nsteps)
 {
     if(nsteps <= 0) {return;}
+    if(c->torn) {throw Error(MJG_ESTATE, "an earlier mjg_step stopped half-way without rollback: mjg_commit first");}
     cudaStream_t st = c->stream;
+    bool stalled = false;                           // the chunk's waits ran out once: step by launches instead
     for(int attempt = 0; attempt < 8; ++attempt)
     {
-        const bool multi = c->graphs && run_fits(c);
+        const bool multi = c->graphs && run_fits(c) && !stalled;
         if(c->rollback && !multi)                   // the multi-step kernel copies the state itself
         {
             CK(cudaMemcpyAsync(c->b_sys.p, c->d_sys.p, c->d_sys.bytes, cudaMemcpyDeviceToDevice, st));
@@ -1552,6 +1568,7 @@ void run_steps(mjg_context* c, int64_t nsteps)
             r.l = c->local;
             r.barrier = c->d_run.as<unsigned>();
             r.disp2 = reinterpret_cast<unsigned long long*>(c->d_run.as<char>() + 256);
+            r.wait_cycles = c->wait_cycles;
             for(int64_t k = 0; k < nsteps; k += RUN_STEPS)
             {
                 r.nsteps = (int)std::min<int64_t>(RUN_STEPS, nsteps - k);
@@ -1584,9 +1601,25 @@ void run_steps(mjg_context* c, int64_t nsteps)
         CK(cudaGetLastError());
         download_sys(c);
         bool overflow = false;
-        check_status(c, overflow);
-        if(!overflow) {return;}
-        if(!c->rollback) {throw Error(MJG_ESTATE, "a Verlet list overflowed (enable rollback)");}
+        if(multi && (c->h_sys[0].status & ST_BARRIER))
+        {
+            stalled = true;                         // whatever else the chunk reports is of a torn step
+            clear_stalled(c);
+            if(!c->rollback)
+            {
+                c->torn = true;
+                rebuild_all(c);
+                CK(cudaStreamSynchronize(st));
+                throw Error(MJG_ECUDA, "a grid barrier of the multi-step kernel ran out of time "
+                                       "(enable rollback to run the steps again)");
+            }
+        }
+        else
+        {
+            check_status(c, overflow);
+            if(!overflow) {return;}
+            if(!c->rollback) {throw Error(MJG_ESTATE, "a Verlet list overflowed (enable rollback)");}
+        }
         // roll back, grow the lists, rebuild, retry
         CK(cudaMemcpyAsync(c->d_sys.p, c->b_sys.p, c->d_sys.bytes, cudaMemcpyDeviceToDevice, st));
         CK(cudaMemcpyAsync(c->d_pos.p, c->b_pos.p, c->d_pos.bytes, cudaMemcpyDeviceToDevice, st));
@@ -1702,6 +1735,14 @@ int mjg_context_set_rollback(mjg_context* c, int enable)
     ABI_BEGIN(c)
     if(c->committed) {throw Error(MJG_ESTATE, "set rollback before mjg_commit");}
     c->rollback = enable != 0;
+    ABI_END(c)
+}
+
+int mjg_context_set_wait_limit(mjg_context* c, int64_t cycles)
+{
+    ABI_BEGIN(c)
+    if(cycles < 0) {throw Error(MJG_EINVAL, "negative wait limit");}
+    c->wait_cycles = cycles > 0 ? cycles : RUN_WAIT_CYCLES;
     ABI_END(c)
 }
 

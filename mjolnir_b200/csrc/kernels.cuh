@@ -163,6 +163,7 @@ void launch_set_force(const Arena& a, const double* src, long long first, long l
 // Many steps of a small arena in one launch (run.cu).
 constexpr int RUN_MAX_SYSTEMS = 64;
 constexpr int RUN_CLUSTER_MAX = 8;   // blocks up to which the launch is one cluster (the portable size)
+constexpr long long RUN_WAIT_CYCLES = 2LL << 30;   // default wait_cycles: about a second
 struct RunArgs {
     Arena a;
     TermArrays t[NGLOBAL];
@@ -175,6 +176,7 @@ struct RunArgs {
     double4* b_vel;
     longlong4* b_force;              // the bits of either form
     double4* b_accel;
+    long long wait_cycles;           // time limit of a wait at the grid barrier
     int nsteps;
     int kick;                        // open with the closing half of the step before this launch
     int close;                       // end with the closing half of the last step

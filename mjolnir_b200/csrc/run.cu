@@ -45,10 +45,10 @@ using ull = unsigned long long;
 // hardware barrier.  Otherwise one word counts arrivals: every block adds 1,
 // block 0 adds what takes the sum to the next multiple of 2^31, and a waiting
 // block watches the top bit flip, so the word needs no reset between barriers
-// or launches.  The wait is bounded in time (BARRIER_CYCLES, about a second): a
-// block that gives up raises ST_BARRIER, and every block returns at its next
-// barrier.
-constexpr long long BARRIER_CYCLES = 2LL << 30;
+// or launches.  The wait is bounded in time (RunArgs::wait_cycles): a block that
+// gives up raises ST_BARRIER, every block returns at its next barrier, and the
+// chunk's later launches return at once, since the word has stopped half-way.
+// The host then clears what the steps left behind (run_steps, context.cu).
 
 // The last warp's first lane arrives and polls: the first warps hold the
 // particles (Grid::warp), whose noise is drawn meanwhile.
@@ -56,6 +56,7 @@ constexpr int POLLER = RT - 32;
 struct Barrier {
     unsigned* word;
     int* status;
+    long long limit;
     bool cluster;
     unsigned old;
     __device__ __forceinline__ void arrive()
@@ -88,7 +89,7 @@ struct Barrier {
             {
                 asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(now) : "l"(word) : "memory");
                 if((old ^ now) & 0x80000000u) {break;}
-                if(clock64() - t0 > BARRIER_CYCLES) {atomicOr(status, ST_BARRIER); ok = 0; break;}
+                if(clock64() - t0 > limit) {atomicOr(status, ST_BARRIER); ok = 0; break;}
             }
         }
         return __syncthreads_and(ok) != 0;
@@ -399,7 +400,7 @@ __global__ void __launch_bounds__(RT, 1) k_run(const __grid_constant__ RunArgs r
     a.sys = sys;
     const int nsys = a.nsys;
     const Grid G;
-    Barrier bar{r.barrier, &r.a.sys[0].status, r.cluster != 0, 0u};
+    Barrier bar{r.barrier, &r.a.sys[0].status, r.wait_cycles, r.cluster != 0, 0u};
     const unsigned full = 0xffffffffu;
     {
         static_assert(sizeof(SysDev) % sizeof(int4) == 0, "copied in 16-byte words");
@@ -413,6 +414,9 @@ __global__ void __launch_bounds__(RT, 1) k_run(const __grid_constant__ RunArgs r
         for(int w = threadIdx.x; w < nsys * NGLOBAL; w += RT) {(&sh.rebuilds[0][0])[w] = 0;}
     }
     __syncthreads();
+    // a wait of an earlier launch of the chunk ran out (the first launch, which
+    // alone writes the rollback copies, never starts with the bit set)
+    if(r.kick && (sys[0].status & ST_BARRIER)) {return;}
     ull* const disp = r.disp2;                    // [2][nsys], zero between launches
 
     // this thread's first particle and its noise, drawn while the grid waits

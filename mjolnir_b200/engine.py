@@ -238,6 +238,9 @@ class Engine:
         t = A.TERM_NAMES.index(term) if isinstance(term, str) else int(term)
         self._c(self.lib.mjg_set_list_capacity(self.ctx, t, int(cap)))
 
+    def debug_set_wait_limit(self, cycles: int):
+        self._c(self.lib.mjg_context_set_wait_limit(self.ctx, int(cycles)))
+
     def stream_handle(self) -> int:
         """cudaStream_t of the context, as an integer (for torch.cuda.ExternalStream)."""
         h = C.c_void_p()
