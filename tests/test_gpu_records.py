@@ -50,3 +50,25 @@ def test_records_equal_separate_terms(kind, n, precision):
     else:
         # sums of at most some ten terms per particle in another order
         assert np.abs(total - want).max() <= 1e-13 * sum(np.abs(p).max() for p in parts) * 10
+
+
+@pytest.mark.parametrize("precision", ["mixed", "fp64"])
+def test_bond_of_exactly_half_a_box(precision):
+    """Two beads exactly half a periodic box apart: the minimum image takes
+    -half a box for the bond's displacement (core/BoundaryCondition.hpp:81-91),
+    and the step's bonded forces have that direction."""
+    d = S.polymer_melt(nchains=1, nbeads=6, radius=40.0, seed=1)
+    d.exv = d.dh = None
+    d.boundary, d.lower, d.upper = "PeriodicCuboid", (-8.0, -8.0, -8.0), (8.0, 8.0, 8.0)
+    d.pos = np.array([[-4.0, 0, 0], [4, 0, 0], [4, -4, 1], [4, 4, 1], [2, 1, 4], [1, 3, -4]], dtype=float)
+    d.bonds = (np.array([[0, 1], [2, 3], [4, 5]]), np.full(3, 10.0), np.full(3, 3.8))
+    d.angles = (np.array([[0, 1, 2], [2, 3, 4]]), np.full(2, 2.0), np.full(2, 1.9))      # these join two of the bonds
+    d.dihedrals = None
+    e = Engine(precision)
+    sid = e.add_system(d)
+    e.commit()
+    total = e.state(sid)[2]
+    bond, angle = (e.term_force(sid, t)[0] for t in ("bond", "angle"))
+    e.close()
+    assert bond[0, 0] < 0 < bond[1, 0]        # pulled together through the boundary: r1 - r0 is -8 there
+    assert np.abs(total - bond - angle).max() <= (0.0 if precision == "mixed" else 1e-12)
