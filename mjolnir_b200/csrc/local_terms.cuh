@@ -517,9 +517,10 @@ __device__ __forceinline__ void record_mixed(const Arena& a, const LocalArrays& 
     if(idx.z >= 0) {W.add_fx(a.force, idx.z, f2.x, f2.y, f2.z);}
     if(term.y >= 0)
     {
-        // its own displacement: the minimum image of a component of exactly half
-        // a box is -half a box from either end, not the negated other one
-        const double3 d = direction(S, p0, p1);
+        double3 d = make_double3(-d10.x, -d10.y, -d10.z);
+        // a component of exactly half a box: its minimum image is -half a box
+        // from either end, not the negated other one
+        if(image_needed(d.x, d.y, d.z, S.halfw_hi)) {d = direction(S, a.pos[idx.x], a.pos[idx.y]);}
         const double c = bond_coefficient(dot(d, d), bkv);
         f0.add(-d.x * c, -d.y * c, -d.z * c);
         f1.add(d.x * c, d.y * c, d.z * c);
