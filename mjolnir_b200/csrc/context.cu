@@ -187,6 +187,7 @@ struct mjg_context {
     mjg::DevBuf b_sys, b_pos, b_vel, b_force, b_accel;   // rollback copies
     mjg::DevBuf d_force_scratch;
     mjg::DevBuf d_run;                      // multi-step kernel: barrier word, displacements
+    mjg::DevBuf d_pair_force;               // multi-step kernel, plain form: each global term's forces
     int sms = 0;                            // SMs of the device
     int64_t wait_cycles = mjg::RUN_WAIT_CYCLES;   // limit of a wait inside the multi-step kernel
     bool torn = false;                      // a chunk stopped half-way and could not be rolled back
@@ -222,7 +223,7 @@ int64_t device_bytes(const mjg_context* c)
     const DevBuf* bufs[] = {&c->d_sys, &c->d_pos, &c->d_vel, &c->d_force, &c->d_coef, &c->d_psys,
                             &c->d_staging, &c->d_mol, &c->b_sys, &c->b_pos, &c->b_vel, &c->b_force,
                             &c->d_accel, &c->b_accel,
-                            &c->d_force_scratch, &c->d_run, &c->l_bond_idx, &c->l_bond_k, &c->l_bond_v0,
+                            &c->d_force_scratch, &c->d_run, &c->d_pair_force, &c->l_bond_idx, &c->l_bond_k, &c->l_bond_v0,
                             &c->l_bond_sys, &c->l_angle_idx, &c->l_angle_k, &c->l_angle_v0,
                             &c->l_angle_sys, &c->l_dihd_idx, &c->l_dihd_k, &c->l_dihd_n,
                             &c->l_dihd_v0, &c->l_dihd_sys, &c->l_win_bond, &c->l_win_angle,
@@ -921,6 +922,17 @@ void make_sysdev(const HostSystem& s, SysDev& d)
     }
 }
 
+// Arenas whose chunks run in the multi-step kernel: there a step's launches and
+// gaps cost more than its work.  Measured (graph of launches / multi-step, us
+// per step): 200 beads 23 / 9.4, 4,096 Lennard-Jones 33 / 17.6, 10,000-bead
+// melt 31 / 14.8, 40 melts of 115,000 beads in all 73 / 71, 262,144-bead fluid
+// 440 / 415 (FP64, untuned shapes), 1,048,576-bead fluid 1150 / 1210 (tuned
+// shapes, which the multi-step kernel has no form of); the line lies where the
+// two meet.
+constexpr long long RUN_MAX_PARTICLES = 131072;
+constexpr int64_t RUN_STEPS = 1024;             // steps per launch
+bool run_fits(long long n, int nsys) {return n > 0 && n <= RUN_MAX_PARTICLES && nsys <= RUN_MAX_SYSTEMS;}
+
 // Packs every live system into one arena and uploads it.  Systems keep their
 // state (positions, velocities, exact forces, step counters) across commits.
 // The host work runs in parallel over systems into one page-locked buffer,
@@ -1201,6 +1213,12 @@ void commit(mjg_context* c)
     c->d_force_scratch.ensure(32 * (size_t)std::max<long long>(n_tot, 1));
     c->d_run.ensure(256 + sizeof(unsigned long long) * 2 * RUN_MAX_SYSTEMS);
     CK(cudaMemsetAsync(c->d_run.p, 0, c->d_run.bytes, st));
+    if(c->precision == P_FP64 && run_fits(n_tot, nsys))
+    {
+        c->d_pair_force.ensure(sizeof(double4) * NGLOBAL * (size_t)n_tot);
+        CK(cudaMemsetAsync(c->d_pair_force.p, 0, c->d_pair_force.bytes, st));   // particles without a slot
+    }
+    else {c->d_pair_force.release();}
     // the per-particle auxiliary array: UnderdampedLangevin accelerations,
     // G-JF coefficients
     bool any_underdamped = false, any_gjf = false;
@@ -1509,20 +1527,6 @@ void check_status(mjg_context* c, bool& overflow)
     }
 }
 
-// Arenas whose chunks run in the multi-step kernel: there a step's launches and
-// gaps cost more than its work.  Measured (graph of launches / multi-step, us
-// per step): 200 beads 23 / 9.4, 4,096 Lennard-Jones 33 / 17.6, 10,000-bead
-// melt 31 / 14.8, 40 melts of 115,000 beads in all 73 / 71, 262,144-bead fluid
-// 440 / 415 (FP64, untuned shapes), 1,048,576-bead fluid 1150 / 1210 (tuned
-// shapes, which the multi-step kernel has no form of); the line lies where the
-// two meet.
-constexpr long long RUN_MAX_PARTICLES = 131072;
-constexpr int64_t RUN_STEPS = 1024;             // steps per launch
-bool run_fits(const mjg_context* c)
-{
-    return c->arena.n > 0 && c->arena.n <= RUN_MAX_PARTICLES && c->arena.nsys <= RUN_MAX_SYSTEMS;
-}
-
 // After a wait inside the multi-step kernel ran out: the arrival word and the
 // displacements, and the counters of a rebuild that stopped between its phases
 // (every rebuild expects them zero; a count left over would send slots past the
@@ -1546,7 +1550,7 @@ void run_steps(mjg_context* c, int64_t nsteps)
     bool stalled = false;                           // the chunk's waits ran out once: step by launches instead
     for(int attempt = 0; attempt < 8; ++attempt)
     {
-        const bool multi = c->graphs && run_fits(c) && !stalled;
+        const bool multi = c->graphs && run_fits(c->arena.n, c->arena.nsys) && !stalled;
         if(c->rollback && !multi)                   // the multi-step kernel copies the state itself
         {
             CK(cudaMemcpyAsync(c->b_sys.p, c->d_sys.p, c->d_sys.bytes, cudaMemcpyDeviceToDevice, st));
@@ -1569,6 +1573,7 @@ void run_steps(mjg_context* c, int64_t nsteps)
             r.barrier = c->d_run.as<unsigned>();
             r.disp2 = reinterpret_cast<unsigned long long*>(c->d_run.as<char>() + 256);
             r.wait_cycles = c->wait_cycles;
+            r.pair_force = c->d_pair_force.as<double4>();
             for(int64_t k = 0; k < nsteps; k += RUN_STEPS)
             {
                 r.nsteps = (int)std::min<int64_t>(RUN_STEPS, nsteps - k);

@@ -28,7 +28,7 @@ __global__ void __launch_bounds__(TPB) k_integrate_first(Arena a)
         SysDev& S = a.sys[s];
         d2 = advance_particle<PREC, AUX>(a, S, i, KICK, S.step, [&](double& r0, double& r1, double& r2) {
             gaussian3(S.seed, (unsigned long long)(i - S.off), S.step, r0, r1, r2);
-        });
+        }, [&](double& fx, double& fy, double& fz) {load_force<PREC>(a.force, i, fx, fy, fz);});
     }
     // per-system maximum: warp-level when the warp sits in one system
     const unsigned full = 0xffffffffu;
@@ -86,7 +86,9 @@ __global__ void __launch_bounds__(TPB) k_integrate_last(Arena a)
     if(i >= a.n) {return;}
     const SysDev& S = a.sys[a.psys[i]];
     if(S.frozen) {return;}
-    close_particle<PREC>(a, S, i, S.step);
+    double fx, fy, fz;
+    load_force<PREC>(a.force, i, fx, fy, fz);
+    close_particle(a, S, i, S.step, fx, fy, fz);
 }
 
 // UnderdampedLangevinIntegrator::initialize (:160-181): a = f/m + sigma R,

@@ -52,18 +52,19 @@ __device__ __forceinline__ void underdamped_close(const SysDev& S, long long i, 
 // coordinates and its force reset; returns its squared displacement.  kick:
 // the previous step's closing half is applied first, as separate rounding
 // steps, so that consecutive steps of a chunk share one pass.  noise(r0, r1,
-// r2) gives the particle's three deviates of this step.  AUX: the arena holds
-// UnderdampedLangevin or G-JF systems (their branches cost registers, and
-// occupancy, in the BAOAB / velocity-Verlet arenas that have none).
-template<int PREC, bool AUX, class NOISE>
+// r2) gives the particle's three deviates of this step, force(fx, fy, fz) its
+// force.  AUX: the arena holds UnderdampedLangevin or G-JF systems (their
+// branches cost registers, and occupancy, in the BAOAB / velocity-Verlet arenas
+// that have none).
+template<int PREC, bool AUX, class NOISE, class FORCE>
 __device__ __forceinline__ double advance_particle(const Arena& a, SysDev& S, long long i, bool kick,
-                                                   unsigned long long step, NOISE&& noise)
+                                                   unsigned long long step, NOISE&& noise, FORCE&& force)
 {
     double4 p = a.pos[i];
     double4 v = a.vel[i];
     const double4 c = S.uniform_coef ? S.coef : a.coef[i];     // per integrator: see Arena::coef
     double fx, fy, fz;
-    load_force<PREC>(a.force, i, fx, fy, fz);
+    force(fx, fy, fz);
     // the particle's slots and their parameters, requested with its state
     int so[NGLOBAL];
     double sw[NGLOBAL];
@@ -196,11 +197,9 @@ __device__ __forceinline__ double advance_particle(const Arena& a, SysDev& S, lo
 
 // The closing half of the last step of a chunk: v += (halfdt/m) f (BAOAB,
 // velocity Verlet, G-JF) or the UnderdampedLangevin closing
-template<int PREC>
-__device__ __forceinline__ void close_particle(const Arena& a, const SysDev& S, long long i, unsigned long long step)
+__device__ __forceinline__ void close_particle(const Arena& a, const SysDev& S, long long i, unsigned long long step,
+                                               double fx, double fy, double fz)
 {
-    double fx, fy, fz;
-    load_force<PREC>(a.force, i, fx, fy, fz);
     double4 v = a.vel[i];
     if(S.integrator == I_UNDERDAMPED)
     {

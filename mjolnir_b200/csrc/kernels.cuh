@@ -170,6 +170,8 @@ struct RunArgs {
     LocalArrays l;
     unsigned* barrier;               // arrival word of the grid barrier (zero before its first use)
     unsigned long long* disp2;       // [2 nsys] largest squared displacements, zero between launches
+    double4* pair_force;             // plain form: [NGLOBAL n] each global term's forces within the launch, zero
+                                     // where a particle has no slot
     // copies of the state before the launch, for a rollback (nullptr: none wanted)
     SysDev* b_sys;
     double4* b_pos;

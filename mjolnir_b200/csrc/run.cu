@@ -113,13 +113,35 @@ struct DirectAdd {
     }
 };
 
-__device__ __forceinline__ void add_force(void* force, long long i, const Acc<P_MIXED>& acc) {acc.store(force, i);}
-// The plain form adds with FP64 atomics here: the terms of one particle land
-// in any order (the launches of a step add them one term after the other).
-__device__ __forceinline__ void add_force(void* force, long long i, const Acc<P_FP64>& acc)
+// A pair term's force on particle i.  The mixed form adds integers, exact in any
+// order.  The plain form keeps each global term's forces apart and whoever reads
+// the particle's force adds them in the order of a step's launches (run_force):
+// FP64 sums by atomics would land in any order, and a run would not repeat.
+__device__ __forceinline__ void put_force(const Arena& a, double4*, long long i, const Acc<P_MIXED>& acc) {acc.store(a.force, i);}
+__device__ __forceinline__ void put_force(const Arena&, double4* pair_force, long long i, const Acc<P_FP64>& acc)
 {
-    double* f = reinterpret_cast<double*>(static_cast<double4*>(force) + i);
-    atomicAdd(f + 0, acc.x); atomicAdd(f + 1, acc.y); atomicAdd(f + 2, acc.z);
+    pair_force[i] = make_double4(acc.x, acc.y, acc.z, 0.0);
+}
+
+// Particle i's force after a step of this launch: in the plain form the bonded
+// terms' sum, then ExcludedVolume, DebyeHuckel and Lennard-Jones (zero where the
+// particle has no slot), all requested together.  whole: the force array holds
+// the whole force, as between launches.
+template<int PREC>
+__device__ __forceinline__ void run_force(const RunArgs& r, bool whole, long long i, double& fx, double& fy, double& fz)
+{
+    load_force<PREC>(r.a.force, i, fx, fy, fz);
+    if constexpr(PREC == P_FP64)
+    {
+        double4 t[NGLOBAL];
+#pragma unroll
+        for(int g = 0; g < NGLOBAL; ++g) {t[g] = load_pd(r.pair_force + g * r.a.n + i);}
+#pragma unroll
+        for(int g = 0; g < NGLOBAL; ++g)
+        {
+            fx += whole ? 0.0 : t[g].x; fy += whole ? 0.0 : t[g].y; fz += whole ? 0.0 : t[g].z;
+        }
+    }
 }
 
 // ------------------------------------------------------------------ rebuild
@@ -283,7 +305,7 @@ __device__ __forceinline__ void clear_cells(const Arena& a, const TermArrays& t,
 // together (every slot owns at least 32 words; those past the length are never
 // used as indices), so the chain is two loads deep: these, then the partners.
 template<int PREC, int G>
-__device__ __forceinline__ void pair_item(const Arena& a, const TermArrays& t, int e)
+__device__ __forceinline__ void pair_item(const Arena& a, const TermArrays& t, double4* pair_force, int e)
 {
     const int lane = threadIdx.x & 31;
     const int tpp = t.tpp, lt = __ffs(tpp) - 1;
@@ -331,7 +353,7 @@ __device__ __forceinline__ void pair_item(const Arena& a, const TermArrays& t, i
         }
     }
     for(int o = tpp / 2; o > 0; o >>= 1) {acc.shfl_add(o);}
-    if(active && lg == 0 && head.n > 0) {add_force(a.force, particle, acc);}
+    if(active && lg == 0 && (PREC == P_FP64 || head.n > 0)) {put_force(a, pair_force, particle, acc);}
     if(ovf) {atomicOr(&a.sys[head.sys].status, ST_FIXED_OVERFLOW);}
 }
 
@@ -379,11 +401,11 @@ __device__ __forceinline__ void forces(const Arena& a, const RunArgs& r, const G
     for(int e = G.warp; e < total; e += G.nwarp)
     {
         int k = e;
-        if(k < n_dh) {pair_item<PREC, G_DH>(a, r.t[G_DH], k); continue;}
+        if(k < n_dh) {pair_item<PREC, G_DH>(a, r.t[G_DH], r.pair_force + G_DH * a.n, k); continue;}
         k -= n_dh;
-        if(k < n_lj) {pair_item<PREC, G_LJ>(a, r.t[G_LJ], k); continue;}
+        if(k < n_lj) {pair_item<PREC, G_LJ>(a, r.t[G_LJ], r.pair_force + G_LJ * a.n, k); continue;}
         k -= n_lj;
-        if(k < n_ex) {pair_item<PREC, G_EXV>(a, r.t[G_EXV], k); continue;}
+        if(k < n_ex) {pair_item<PREC, G_EXV>(a, r.t[G_EXV], r.pair_force + G_EXV * a.n, k); continue;}
         local_item<PREC>(a, r.l, k - n_ex);
     }
 }
@@ -452,7 +474,7 @@ __global__ void __launch_bounds__(RT, 1) k_run(const __grid_constant__ RunArgs r
                 d2 = advance_particle<PREC, AUX>(a, S, i, k > 0 || r.kick, step, [&](double& x, double& y, double& z) {
                     if(i == i0) {x = n0; y = n1; z = n2;}
                     else        {gaussian3(S.seed, (ull)(i - S.off), step, x, y, z);}
-                });
+                }, [&](double& fx, double& fy, double& fz) {run_force<PREC>(r, k == 0, i, fx, fy, fz);});
             }
             const int s0 = __shfl_sync(full, s, 0);
             if(__all_sync(full, s == s0 || s < 0))
@@ -499,13 +521,17 @@ __global__ void __launch_bounds__(RT, 1) k_run(const __grid_constant__ RunArgs r
         draw(k + 1);                              // while the others finish
         if(!bar.wait()) {return;}
     }
-    // ---- closing half of the last step, counters
-    if(r.close)
+    // ---- the whole force, closing half of the last step, counters
+    if(r.close || PREC == P_FP64)
     {
         for(long long i = i0; i < a.n; i += G.nthread)
         {
             const int s = a.psys[i];
-            if(!sys[s].frozen) {close_particle<PREC>(a, sys[s], i, sys[s].step + r.nsteps);}
+            if(sys[s].frozen) {continue;}
+            double fx, fy, fz;
+            run_force<PREC>(r, false, i, fx, fy, fz);
+            if constexpr(PREC == P_FP64) {static_cast<double4*>(a.force)[i] = make_double4(fx, fy, fz, 0.0);}
+            if(r.close) {close_particle(a, sys[s], i, sys[s].step + r.nsteps, fx, fy, fz);}
         }
     }
     __syncthreads();

@@ -89,3 +89,26 @@ def test_half_lists_and_frozen_systems(half, frozen):
         assert g[1] == w[1] and g[2] == w[2]
         for x, y in zip(g[0], w[0]):
             assert np.array_equal(x, y)
+
+
+@pytest.mark.parametrize("graphs", [True, False])
+def test_fp64_runs_repeat(graphs):
+    """FP64 sums that no launch leaves to the order of arrival repeat bit for bit: three pair terms on one
+    particle, and pair terms beside at most two bonds."""
+    three = S.bead_fluid(n=1500, density=0.003, seed=33, dt=0.6, margin=0.1)
+    lj = S.lj_fluid(n=343, seed=32, margin=0.05)
+    three.lj = lj.lj
+    three.lj.idx = np.arange(three.n)
+    three.lj.param0, three.lj.param1 = np.full(three.n, 4.0), np.full(three.n, 0.3)
+    bonded = S.polymer_melt(nchains=9, nbeads=111, radius=55.0, seed=5, margin=0.15)
+    bonded.angles = bonded.dihedrals = None
+    outs = []
+    for _ in range(3):
+        e = Engine("fp64", graphs=graphs)
+        ids = [e.add_system(d) for d in (three, bonded)]
+        e.commit()
+        e.step(300)
+        outs.append([x for sid in ids for x in e.state(sid)])
+        e.close()
+    for o in outs[1:]:
+        assert all(np.array_equal(x, y) for x, y in zip(o, outs[0]))
