@@ -63,7 +63,8 @@ MJG_API int  mjg_context_create(int device, int precision, mjg_context** out);
 MJG_API void mjg_context_destroy(mjg_context* ctx);
 MJG_API const char* mjg_last_error(const mjg_context* ctx);
 /* 1 (default): mjg_step replays captured CUDA graphs of the step, or, in a
- * small arena, runs many steps in one cooperative launch; 0: it launches every
+ * small arena, runs up to 1,024 steps in one cooperative launch, which holds
+ * the SMs it runs on until it ends (about 10 ms at most); 0: it launches every
  * kernel of every step. */
 MJG_API int  mjg_context_set_graphs(mjg_context* ctx, int enable);
 /* Options: the per-step work of mjg_step is also checked for list overflow

@@ -930,7 +930,14 @@ void make_sysdev(const HostSystem& s, SysDev& d)
 // shapes, which the multi-step kernel has no form of); the line lies where the
 // two meet.
 constexpr long long RUN_MAX_PARTICLES = 131072;
-constexpr int64_t RUN_STEPS = 1024;             // steps per launch
+// Steps per launch.  A launch holds every SM it runs on until it ends, so this
+// bounds how long other work on the GPU waits: about 10 ms (200 beads 1,024 steps
+// of 8 us, 10,000-bead melt 838 of 12, 115,000 beads 72 of 55 to 150).  A launch
+// costs 10 to 20 us beside its steps: 128 steps each were 1 % slower at 200 beads.
+int64_t run_steps_per_launch(long long n)
+{
+    return std::min<int64_t>(1024, std::max<int64_t>(64, (1LL << 23) / n));
+}
 bool run_fits(long long n, int nsys) {return n > 0 && n <= RUN_MAX_PARTICLES && nsys <= RUN_MAX_SYSTEMS;}
 
 // Packs every live system into one arena and uploads it.  Systems keep their
@@ -1574,9 +1581,10 @@ void run_steps(mjg_context* c, int64_t nsteps)
             r.disp2 = reinterpret_cast<unsigned long long*>(c->d_run.as<char>() + 256);
             r.wait_cycles = c->wait_cycles;
             r.pair_force = c->d_pair_force.as<double4>();
-            for(int64_t k = 0; k < nsteps; k += RUN_STEPS)
+            const int64_t per_launch = run_steps_per_launch(c->arena.n);
+            for(int64_t k = 0; k < nsteps; k += per_launch)
             {
-                r.nsteps = (int)std::min<int64_t>(RUN_STEPS, nsteps - k);
+                r.nsteps = (int)std::min<int64_t>(per_launch, nsteps - k);
                 r.kick = k > 0 ? 1 : 0;
                 const bool copy = c->rollback && k == 0;
                 r.b_sys = copy ? c->b_sys.as<SysDev>() : nullptr;

@@ -112,3 +112,44 @@ def test_fp64_runs_repeat(graphs):
         e.close()
     for o in outs[1:]:
         assert all(np.array_equal(x, y) for x, y in zip(o, outs[0]))
+
+
+@pytest.mark.parametrize("name,per_launch", [("chain_33", 1024), ("integrators", 1024), ("fluid_40001", 209)])
+def test_chunks_of_several_launches(name, per_launch):
+    """A chunk longer than a launch: the closing half of the step before opens the next launch, and the step
+    counters, margins and displacements carry over."""
+    steps = (per_launch, per_launch + 1, 2 * per_launch + 17)
+    got, few = run(name, "mixed", True, steps=steps)
+    want, _ = run(name, "mixed", False, steps=steps)
+    assert few == 1 + 2 + 3
+    for g, w in zip(got, want):
+        assert g[1] == w[1] and g[2] == w[2]
+        assert all(np.array_equal(x, y) for x, y in zip((*g[0], *g[3]), (*w[0], *w[3])))
+
+
+def test_overflow_in_a_later_launch_rolls_the_chunk_back():
+    """A list that outgrows its capacity only in the second launch of a chunk or later: the copy that the first
+    launch took is restored, with the accelerations of UnderdampedLangevin and the coefficients of G-JF."""
+    descs = [S.lj_fluid(n=1000, density=0.3, margin=0.05, seed=44 + k) for k in range(3)]      # condenses
+    for d, kind in zip(descs, ("UnderdampedLangevin", "G-JFLangevin", "BAOAB")):
+        d.integrator = kind
+
+    def states(steps, cap=None):
+        e = Engine("mixed")
+        ids = [e.add_system(d) for d in descs]
+        e.commit()
+        if cap:
+            e.debug_set_list_capacity("lj", cap)
+        n0 = e.launch_count()
+        e.step(steps)
+        launches = e.launch_count() - n0
+        out = [x for sid in ids for x in e.state(sid)]
+        e.close()
+        return out, launches
+
+    # the smallest capacity that the first launch's lists keep within
+    cap = next(c for c in range(24, 129) if states(1024, c)[1] == 1)
+    want, plain = states(5000)
+    got, redone = states(5000, cap)
+    assert plain == 5 and redone > 5
+    assert all(np.array_equal(x, y) for x, y in zip(got, want))
