@@ -1534,7 +1534,7 @@ void check_status(mjg_context* c, bool& overflow)
     }
 }
 
-// After a wait inside the multi-step kernel ran out: the arrival word and the
+// After a wait inside the multi-step kernel ran out: the barrier words and the
 // displacements, and the counters of a rebuild that stopped between its phases
 // (every rebuild expects them zero; a count left over would send slots past the
 // term's arrays).

@@ -163,12 +163,14 @@ void launch_set_force(const Arena& a, const double* src, long long first, long l
 // Many steps of a small arena in one launch (run.cu).
 constexpr int RUN_MAX_SYSTEMS = 64;
 constexpr int RUN_CLUSTER_MAX = 8;   // blocks up to which the launch is one cluster (the portable size)
+constexpr int RUN_LEFT = 32;         // in a line of its own
 constexpr long long RUN_WAIT_CYCLES = 2LL << 30;   // default wait_cycles: about a second
 struct RunArgs {
     Arena a;
     TermArrays t[NGLOBAL];
     LocalArrays l;
-    unsigned* barrier;               // arrival word of the grid barrier (zero before its first use)
+    unsigned* barrier;               // words of the grid barrier: [0] arrivals, [RUN_LEFT] blocks that have
+                                     // left, both zero between launches
     unsigned long long* disp2;       // [2 nsys] largest squared displacements, zero between launches
     double4* pair_force;             // plain form: [NGLOBAL n] each global term's forces within the launch, zero
                                      // where a particle has no slot

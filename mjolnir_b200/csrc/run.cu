@@ -42,26 +42,24 @@ using ull = unsigned long long;
 
 // ------------------------------------------------------------------ barrier
 // All blocks of the grid.  A launch that fits one cluster uses the cluster's
-// hardware barrier.  Otherwise one word counts arrivals: every block adds 1,
-// block 0 adds what takes the sum to the next multiple of 2^31, and a waiting
-// block watches the top bit flip, so the word needs no reset between barriers
-// or launches.  The wait is bounded in time (RunArgs::wait_cycles): a block that
-// gives up raises ST_BARRIER, every block returns at its next barrier, and the
-// chunk's later launches return at once, since the word has stopped half-way.
-// The host then clears what the steps left behind (run_steps, context.cu).
+// hardware barrier.  Otherwise a word counts the launch's arrivals: barrier e (from
+// 1) is complete when it has reached e times the number of blocks.  A second word
+// counts the blocks that have left the last barrier, and the last of them sets
+// both back to zero for the next launch.  The wait is bounded in time
+// (RunArgs::wait_cycles): a block that gives up raises ST_BARRIER, every block
+// returns at its next barrier, and the chunk's later launches return at once, since
+// the words have stopped half-way.  The host then clears what the steps left
+// behind (run_steps, context.cu).
 
 // The last warp's first lane arrives and polls: the first warps hold the
 // particles (Grid::warp), whose noise is drawn meanwhile.
 constexpr int POLLER = RT - 32;
 struct Barrier {
-    unsigned* word;
-    int* status;
-    long long limit;
-    bool cluster;
-    unsigned old;
+    const RunArgs& r;
+    unsigned due;                            // arrivals that complete the current barrier
     __device__ __forceinline__ void arrive()
     {
-        if(cluster)
+        if(r.cluster)
         {
             asm volatile("barrier.cluster.arrive.release;" ::: "memory");
             return;
@@ -69,13 +67,13 @@ struct Barrier {
         __syncthreads();
         if(threadIdx.x == POLLER)
         {
-            const unsigned add = blockIdx.x == 0 ? 0x80000000u - (gridDim.x - 1) : 1u;
-            asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], %2;" : "=r"(old) : "l"(word), "r"(add) : "memory");
+            due += gridDim.x;
+            asm volatile("red.release.gpu.global.add.u32 [%0], 1;" :: "l"(r.barrier) : "memory");
         }
     }
     __device__ __forceinline__ bool wait()
     {
-        if(cluster)
+        if(r.cluster)
         {
             asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
             return true;
@@ -83,18 +81,28 @@ struct Barrier {
         int ok = 1;
         if(threadIdx.x == POLLER)
         {
-            unsigned now;
             const long long t0 = clock64();
             for(;;)
             {
-                asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(now) : "l"(word) : "memory");
-                if((old ^ now) & 0x80000000u) {break;}
-                if(clock64() - t0 > limit) {atomicOr(status, ST_BARRIER); ok = 0; break;}
+                unsigned arrived;
+                asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(arrived) : "l"(r.barrier) : "memory");
+                if(arrived >= due) {break;}
+                if(clock64() - t0 > r.wait_cycles) {atomicOr(&r.a.sys[0].status, ST_BARRIER); ok = 0; break;}
             }
         }
         return __syncthreads_and(ok) != 0;
     }
     __device__ __forceinline__ bool sync() {arrive(); return wait();}
+    // after the launch's last barrier
+    __device__ __forceinline__ void leave()
+    {
+        if(r.cluster || threadIdx.x != POLLER) {return;}
+        if(atomicAdd(r.barrier + RUN_LEFT, 1u) == gridDim.x - 1)
+        {
+            r.barrier[0] = 0;
+            r.barrier[RUN_LEFT] = 0;
+        }
+    }
 };
 
 // ------------------------------------------------- bonded forces, one by one
@@ -422,7 +430,7 @@ __global__ void __launch_bounds__(RT, 1) k_run(const __grid_constant__ RunArgs r
     a.sys = sys;
     const int nsys = a.nsys;
     const Grid G;
-    Barrier bar{r.barrier, &r.a.sys[0].status, r.wait_cycles, r.cluster != 0, 0u};
+    Barrier bar{r, 0u};
     const unsigned full = 0xffffffffu;
     {
         static_assert(sizeof(SysDev) % sizeof(int4) == 0, "copied in 16-byte words");
@@ -521,6 +529,7 @@ __global__ void __launch_bounds__(RT, 1) k_run(const __grid_constant__ RunArgs r
         draw(k + 1);                              // while the others finish
         if(!bar.wait()) {return;}
     }
+    bar.leave();
     // ---- the whole force, closing half of the last step, counters
     if(r.close || PREC == P_FP64)
     {
