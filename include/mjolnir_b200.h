@@ -77,6 +77,11 @@ MJG_API int  mjg_context_set_rollback(mjg_context* ctx, int enable);
  * MJG_ECUDA, the particles may be a step apart, and further steps are refused
  * until mjg_commit.  Used to test that path. */
 MJG_API int  mjg_context_set_wait_limit(mjg_context* ctx, int64_t cycles);
+/* Blocks of that launch (0: by the arena's size, at most one per SM).  A
+ * launch that the CUDA runtime refuses, for instance with more blocks than fit
+ * the GPU at once, is replaced by the captured graphs until the next
+ * mjg_commit.  Used to test that path. */
+MJG_API int  mjg_context_set_run_blocks(mjg_context* ctx, int blocks);
 /* Reserves the page-locked host buffers that commits pack into for an
  * arena of up to `particles` particles (about 490 bytes per particle), so
  * that a server which fills its arena over many commits does not page-lock

@@ -32,6 +32,7 @@ SIGNATURES = {
     "mjg_context_set_graphs": (C.c_int, [_ctx, C.c_int]),
     "mjg_context_set_rollback": (C.c_int, [_ctx, C.c_int]),
     "mjg_context_set_wait_limit": (C.c_int, [_ctx, C.c_int64]),
+    "mjg_context_set_run_blocks": (C.c_int, [_ctx, C.c_int]),
     "mjg_system_create": (C.c_int, [_ctx, C.c_int64, C.c_int, _f64p, _f64p, _f64p, _f64p, _f64p,
                                     C.POINTER(C.c_int)]),
     "mjg_system_set_attributes": (C.c_int, [_ctx, C.c_int, C.c_double, C.c_double]),

@@ -190,6 +190,8 @@ struct mjg_context {
     mjg::DevBuf d_pair_force;               // multi-step kernel, plain form: each global term's forces
     int sms = 0;                            // SMs of the device
     int64_t wait_cycles = mjg::RUN_WAIT_CYCLES;   // limit of a wait inside the multi-step kernel
+    int run_blocks = 0;                     // blocks of the multi-step kernel, 0: by the arena's size
+    bool run_refused = false;               // the runtime refused its launch: this arena steps by graphs
     bool torn = false;                      // a chunk stopped half-way and could not be rolled back
     double* h_pinned = nullptr;             // page-locked host staging (state, forces)
     size_t h_pinned_bytes = 0;
@@ -1427,6 +1429,7 @@ void commit(mjg_context* c)
 
     c->committed = true;
     c->torn = false;
+    c->run_refused = false;
     rebuild_all(c);
     tm.mark("rebuild");
     compute_initial_forces(c);
@@ -1557,7 +1560,7 @@ void run_steps(mjg_context* c, int64_t nsteps)
     bool stalled = false;                           // the chunk's waits ran out once: step by launches instead
     for(int attempt = 0; attempt < 8; ++attempt)
     {
-        const bool multi = c->graphs && run_fits(c->arena.n, c->arena.nsys) && !stalled;
+        const bool multi = c->graphs && run_fits(c->arena.n, c->arena.nsys) && !stalled && !c->run_refused;
         if(c->rollback && !multi)                   // the multi-step kernel copies the state itself
         {
             CK(cudaMemcpyAsync(c->b_sys.p, c->d_sys.p, c->d_sys.bytes, cudaMemcpyDeviceToDevice, st));
@@ -1580,6 +1583,7 @@ void run_steps(mjg_context* c, int64_t nsteps)
             r.barrier = c->d_run.as<unsigned>();
             r.disp2 = reinterpret_cast<unsigned long long*>(c->d_run.as<char>() + 256);
             r.wait_cycles = c->wait_cycles;
+            r.blocks = c->run_blocks;
             r.pair_force = c->d_pair_force.as<double4>();
             const int64_t per_launch = run_steps_per_launch(c->arena.n);
             for(int64_t k = 0; k < nsteps; k += per_launch)
@@ -1593,8 +1597,17 @@ void run_steps(mjg_context* c, int64_t nsteps)
                 r.b_force = copy ? c->b_force.as<longlong4>() : nullptr;
                 r.b_accel = copy ? c->b_accel.as<double4>() : nullptr;
                 r.close = k + r.nsteps == nsteps ? 1 : 0;
-                CK(launch_run(r, c->sms, st));
+                const cudaError_t e = launch_run(r, c->sms, st);
+                if(k == 0 && (e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorLaunchOutOfResources ||
+                              e == cudaErrorNotSupported || e == cudaErrorInvalidConfiguration))
+                {
+                    cudaGetLastError();             // refused, nothing has run
+                    c->run_refused = true;
+                    break;
+                }
+                CK(e);
             }
+            if(c->run_refused) {continue;}
         }
         else if(c->graphs)
         {
@@ -1756,6 +1769,15 @@ int mjg_context_set_wait_limit(mjg_context* c, int64_t cycles)
     ABI_BEGIN(c)
     if(cycles < 0) {throw Error(MJG_EINVAL, "negative wait limit");}
     c->wait_cycles = cycles > 0 ? cycles : RUN_WAIT_CYCLES;
+    ABI_END(c)
+}
+
+int mjg_context_set_run_blocks(mjg_context* c, int blocks)
+{
+    ABI_BEGIN(c)
+    if(blocks < 0) {throw Error(MJG_EINVAL, "negative block count");}
+    c->run_blocks = blocks;
+    c->run_refused = false;
     ABI_END(c)
 }
 

@@ -184,8 +184,11 @@ struct RunArgs {
     int nsteps;
     int kick;                        // open with the closing half of the step before this launch
     int close;                       // end with the closing half of the last step
+    int blocks;                      // blocks of the launch; 0: by the size of the force phase
     int cluster;                     // set by the launch: the grid is one cluster
 };
+// An error leaves nothing enqueued (more blocks than can be resident together, a
+// partitioned GPU).
 cudaError_t launch_run(RunArgs r, int sms, cudaStream_t s);
 
 // kernel launch accounting (every wrapper reports what it enqueued)

@@ -570,7 +570,7 @@ cudaError_t launch_run(RunArgs r, int sms, cudaStream_t s)
     for(int g = 0; g < NGLOBAL; ++g) {items += pair_items(r.t[g]);}
     items += local_items(r.a.precision, r.l);
     items = std::max(items, warps_of(r.a.n));
-    int blocks = std::max(1, std::min(sms, (items + RT / 32 - 1) / (RT / 32)));
+    const int blocks = r.blocks > 0 ? r.blocks : std::max(1, std::min(sms, (items + RT / 32 - 1) / (RT / 32)));
     r.cluster = blocks <= RUN_CLUSTER_MAX ? 1 : 0;
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(blocks);
@@ -597,8 +597,9 @@ cudaError_t launch_run(RunArgs r, int sms, cudaStream_t s)
     const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                (int)(sizeof(SysDev) * RUN_MAX_SYSTEMS));
     if(e != cudaSuccess) {return e;}
-    note_launches(1);
-    return cudaLaunchKernelEx(&cfg, kernel, r);
+    const cudaError_t launched = cudaLaunchKernelEx(&cfg, kernel, r);
+    if(launched == cudaSuccess) {note_launches(1);}
+    return launched;
 }
 
 }  // namespace mjg

@@ -241,6 +241,9 @@ class Engine:
     def debug_set_wait_limit(self, cycles: int):
         self._c(self.lib.mjg_context_set_wait_limit(self.ctx, int(cycles)))
 
+    def debug_set_run_blocks(self, blocks: int):
+        self._c(self.lib.mjg_context_set_run_blocks(self.ctx, int(blocks)))
+
     def stream_handle(self) -> int:
         """cudaStream_t of the context, as an integer (for torch.cuda.ExternalStream)."""
         h = C.c_void_p()

@@ -1,8 +1,9 @@
-"""A wait between the blocks of the multi-step kernel that runs out of time (a
-limit of one clock cycle, which nearly every wait exceeds): the chunk is rolled
-back and steps by launches, with the same bits, and nothing of the interrupted
-steps reaches later ones; without rollback the context refuses to step until
-the next commit."""
+"""What stops the multi-step kernel.  A wait between its blocks that runs out of
+time (a limit of one clock cycle, which nearly every wait exceeds): the chunk is
+rolled back and steps by launches, with the same bits, and nothing of the
+interrupted steps reaches later ones; without rollback the context refuses to
+step until the next commit.  A launch that the runtime refuses: the arena steps
+by captured graphs."""
 import numpy as np
 import pytest
 
@@ -83,5 +84,25 @@ def test_without_rollback_steps_are_refused_until_commit():
     ref.step(25)
     for x, y in zip(states(e, ids), states(ref, rid)):
         assert np.array_equal(x, y)
+    e.close()
+    ref.close()
+
+
+@pytest.mark.parametrize("rollback", [True, False])
+def test_refused_launch_steps_by_graphs(rollback):
+    """More blocks than any GPU holds at once: the runtime returns an error and launches nothing."""
+    ref, rid = engine("integrators", graphs=False)
+    e, ids = engine("integrators", rollback=rollback)
+    for k, blocks in ((5, 0), (40, 1 << 20), (30, 1 << 20), (40, 0), (20, 3), (20, 11)):   # 3: one small cluster
+        e.debug_set_run_blocks(blocks)
+        n0 = e.launch_count()
+        e.step(k)
+        assert (e.launch_count() - n0 == 1) == (blocks < 100)
+        ref.step(k)
+        for x, y in zip(states(e, ids), states(ref, rid)):
+            assert np.array_equal(x, y), (k, blocks)
+    e.debug_set_run_blocks(1 << 20)
+    e.step(1)
+    e.debug_set_run_blocks(0)
     e.close()
     ref.close()
