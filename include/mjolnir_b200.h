@@ -64,9 +64,12 @@ MJG_API void mjg_context_destroy(mjg_context* ctx);
 MJG_API const char* mjg_last_error(const mjg_context* ctx);
 /* 1 (default): mjg_step replays captured CUDA graphs of the step, or, in a
  * small arena, runs up to 1,024 steps in one cooperative launch, which holds
- * the SMs it runs on until it ends (about 10 ms at most); 0: it launches every
- * kernel of every step. */
+ * the SMs it runs on until it ends (about 10 ms at most); 2: it replays captured
+ * graphs in small arenas too; 0: it launches every kernel of every step. */
 MJG_API int  mjg_context_set_graphs(mjg_context* ctx, int enable);
+/* How mjg_step runs the committed arena: 0 separate launches, 1 captured
+ * graphs, 2 many steps in one launch. */
+MJG_API int  mjg_context_step_path(mjg_context* ctx, int* path);
 /* Options: the per-step work of mjg_step is also checked for list overflow
  * and rolled back when it happens (default 1). */
 MJG_API int  mjg_context_set_rollback(mjg_context* ctx, int enable);

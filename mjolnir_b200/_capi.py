@@ -30,6 +30,7 @@ SIGNATURES = {
     "mjg_context_destroy": (None, [_ctx]),
     "mjg_last_error": (C.c_char_p, [_ctx]),
     "mjg_context_set_graphs": (C.c_int, [_ctx, C.c_int]),
+    "mjg_context_step_path": (C.c_int, [_ctx, C.POINTER(C.c_int)]),
     "mjg_context_set_rollback": (C.c_int, [_ctx, C.c_int]),
     "mjg_context_set_wait_limit": (C.c_int, [_ctx, C.c_int64]),
     "mjg_context_set_run_blocks": (C.c_int, [_ctx, C.c_int]),

@@ -166,7 +166,7 @@ struct TermDev {
 struct mjg_context {
     int device = 0;
     int precision = mjg::P_FP64;
-    bool graphs = true;
+    int graphs = 1;              // 0 launches, 1 captured graphs or the multi-step kernel, 2 captured graphs
     bool rollback = true;
     cudaStream_t stream = nullptr;
     // branches of the step: one per global term (rebuild, forces) and one for
@@ -1552,6 +1552,11 @@ void clear_stalled(mjg_context* c)
     }
 }
 
+bool steps_in_one_launch(const mjg_context* c)
+{
+    return c->graphs == 1 && run_fits(c->arena.n, c->arena.nsys) && !c->run_refused;
+}
+
 void run_steps(mjg_context* c, int64_t nsteps)
 {
     if(nsteps <= 0) {return;}
@@ -1560,7 +1565,7 @@ void run_steps(mjg_context* c, int64_t nsteps)
     bool stalled = false;                           // the chunk's waits ran out once: step by launches instead
     for(int attempt = 0; attempt < 8; ++attempt)
     {
-        const bool multi = c->graphs && run_fits(c->arena.n, c->arena.nsys) && !stalled && !c->run_refused;
+        const bool multi = steps_in_one_launch(c) && !stalled;
         if(c->rollback && !multi)                   // the multi-step kernel copies the state itself
         {
             CK(cudaMemcpyAsync(c->b_sys.p, c->d_sys.p, c->d_sys.bytes, cudaMemcpyDeviceToDevice, st));
@@ -1751,8 +1756,17 @@ const char* mjg_last_error(const mjg_context* c) {return c ? c->err.c_str() : "n
 int mjg_context_set_graphs(mjg_context* c, int enable)
 {
     ABI_BEGIN(c)
-    c->graphs = enable != 0;
+    c->graphs = enable == 2 ? 2 : (enable != 0 ? 1 : 0);
     release_graph(c);
+    ABI_END(c)
+}
+
+int mjg_context_step_path(mjg_context* c, int* path)
+{
+    ABI_BEGIN(c)
+    if(!path) {throw Error(MJG_EINVAL, "path is NULL");}
+    if(!c->committed) {throw Error(MJG_ESTATE, "mjg_commit first");}
+    *path = steps_in_one_launch(c) ? 2 : (c->graphs ? 1 : 0);
     ABI_END(c)
 }
 

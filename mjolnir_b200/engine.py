@@ -35,7 +35,8 @@ class Engine:
         self.ctx = h
         self.precision = precision
         self.n_of = {}
-        A.check(self.ctx, self.lib.mjg_context_set_graphs(self.ctx, 1 if graphs else 0))
+        # True: captured graphs, or many steps in one launch in a small arena; 2: captured graphs in any arena
+        A.check(self.ctx, self.lib.mjg_context_set_graphs(self.ctx, 2 if graphs == 2 else 1 if graphs else 0))
         A.check(self.ctx, self.lib.mjg_context_set_rollback(self.ctx, 1 if rollback else 0))
 
     def reserve(self, particles: int):
@@ -146,6 +147,12 @@ class Engine:
 
     def commit(self):
         self._c(self.lib.mjg_commit(self.ctx))
+
+    def step_path(self) -> int:
+        """How step() runs the committed arena: 0 separate launches, 1 captured graphs, 2 many steps in one launch."""
+        p = C.c_int()
+        self._c(self.lib.mjg_context_step_path(self.ctx, C.byref(p)))
+        return p.value
 
     def step(self, nsteps: int = 1):
         self._c(self.lib.mjg_step(self.ctx, int(nsteps)))
