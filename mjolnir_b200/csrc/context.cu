@@ -925,22 +925,31 @@ void make_sysdev(const HostSystem& s, SysDev& d)
 }
 
 // Arenas whose chunks run in the multi-step kernel: there a step's launches and
-// gaps cost more than its work.  Measured (graph of launches / multi-step, us
-// per step): 200 beads 23 / 9.4, 4,096 Lennard-Jones 33 / 17.6, 10,000-bead
-// melt 31 / 14.8, 40 melts of 115,000 beads in all 73 / 71, 262,144-bead fluid
-// 440 / 415 (FP64, untuned shapes), 1,048,576-bead fluid 1150 / 1210 (tuned
-// shapes, which the multi-step kernel has no form of); the line lies where the
-// two meet.
-constexpr long long RUN_MAX_PARTICLES = 131072;
+// gaps cost more than its work.  Measured, us per step, graph of launches /
+// multi-step, default launch shapes:
+//   mixed   Lennard-Jones 50,000 75 / 71, 91,000 107 / 111, 118,000 134 / 146;
+//           fluid 60,000 83 / 77, 90,000 122 / 125, 115,000 138 / 148;
+//           melt 10,000 24 / 12, 75,000 37 / 35, 90,000 41 / 42, 115,000 50 / 56;
+//           40 melts 72,000 47 / 41, 88,000 52 / 47, 96,000 51 / 51, 112,000 55 / 56
+//   FP64    Lennard-Jones 118,000 134 / 131, 176,000 189 / 188; fluid 115,000 182 / 165,
+//           180,000 264 / 253, 262,000 361 / 360; melt 115,000 76 / 66, 180,000 99 / 100
+// The mixed form's line lies where the two meet.  The FP64 form's meet later, near
+// 180,000 particles, but the gain is 2 to 13 % at the line and each launch holds
+// the whole GPU.  The number of systems is bounded by the kernel's flag word.
+long long run_max_particles(int precision) {return precision == P_MIXED ? 90000 : 131072;}
+bool run_fits(long long n, int nsys, int precision)
+{
+    return n > 0 && n <= run_max_particles(precision) && nsys <= RUN_MAX_SYSTEMS;
+}
+
 // Steps per launch.  A launch holds every SM it runs on until it ends, so this
 // bounds how long other work on the GPU waits: about 10 ms (200 beads 1,024 steps
-// of 8 us, 10,000-bead melt 838 of 12, 115,000 beads 72 of 55 to 150).  A launch
+// of 8 us, 10,000-bead melt 838 of 12, 90,000 beads 93 of 42 to 125).  A launch
 // costs 10 to 20 us beside its steps: 128 steps each were 1 % slower at 200 beads.
 int64_t run_steps_per_launch(long long n)
 {
     return std::min<int64_t>(1024, std::max<int64_t>(64, (1LL << 23) / n));
 }
-bool run_fits(long long n, int nsys) {return n > 0 && n <= RUN_MAX_PARTICLES && nsys <= RUN_MAX_SYSTEMS;}
 
 // Packs every live system into one arena and uploads it.  Systems keep their
 // state (positions, velocities, exact forces, step counters) across commits.
@@ -1222,7 +1231,7 @@ void commit(mjg_context* c)
     c->d_force_scratch.ensure(32 * (size_t)std::max<long long>(n_tot, 1));
     c->d_run.ensure(256 + sizeof(unsigned long long) * 2 * RUN_MAX_SYSTEMS);
     CK(cudaMemsetAsync(c->d_run.p, 0, c->d_run.bytes, st));
-    if(c->precision == P_FP64 && run_fits(n_tot, nsys))
+    if(c->precision == P_FP64 && run_fits(n_tot, nsys, P_FP64))
     {
         c->d_pair_force.ensure(sizeof(double4) * NGLOBAL * (size_t)n_tot);
         CK(cudaMemsetAsync(c->d_pair_force.p, 0, c->d_pair_force.bytes, st));   // particles without a slot
@@ -1554,7 +1563,7 @@ void clear_stalled(mjg_context* c)
 
 bool steps_in_one_launch(const mjg_context* c)
 {
-    return c->graphs == 1 && run_fits(c->arena.n, c->arena.nsys) && !c->run_refused;
+    return c->graphs == 1 && run_fits(c->arena.n, c->arena.nsys, c->precision) && !c->run_refused;
 }
 
 void run_steps(mjg_context* c, int64_t nsteps)

@@ -76,3 +76,22 @@ def test_launch_shapes_fp64(graphs):
             # rounding of the sums' order, as in the parity test of the launch shapes (velocities and forces react
             # more strongly than positions: the steepest pair potential's relative slope is some 1e2)
             assert np.abs(x - y).max() <= 1e-7 * max(1.0, np.abs(y).max()), shape
+
+
+def test_the_line_between_the_paths():
+    """At the largest arena that steps in one launch, and one particle above it."""
+    for precision, n, path in (("mixed", 90000, 2), ("mixed", 90001, 1), ("fp64", 90001, 2)):
+        d = S.bead_fluid(n=n, density=0.003, seed=8, dt=0.6, margin=0.05)
+        outs = []
+        for graphs in (True, False):
+            e = Engine(precision, graphs=graphs)
+            sid = e.add_system(d)
+            e.commit()
+            if graphs:
+                assert e.step_path() == path
+            e.step(15)
+            assert e.rebuild_count(sid, "exv") > 0
+            outs.append(e.state(sid))
+            e.close()
+        for x, y in zip(*outs):
+            assert np.array_equal(x, y) if precision == "mixed" else np.abs(x - y).max() <= 1e-9 * np.abs(y).max()
