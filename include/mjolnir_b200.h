@@ -282,7 +282,11 @@ MJG_API int mjg_context_get_stream(mjg_context* ctx, void** stream);
  * buffers. */
 MJG_API int mjg_time_kernel(mjg_context* ctx, int term, int reps, double* ms_per_launch);
 /* Performance knobs of a global term (they change no result in the mixed
- * form, whose force sums are exact and order independent):
+ * form, whose force sums are exact and order independent).  An arena that runs
+ * many steps in one launch (mjg_context_step_path 2) honours the threads per
+ * particle, half lists, the margin, the list layout of schedule 5, and of the
+ * build lanes 8 (for 4 and 8) or 32 (for 16 and 32); its steps run no pair
+ * launches, so the batch depth and the rest of the schedule have no effect there.
  * threads cooperating on one particle's list in the pair kernel (1, 2, 4, 8,
  * 16 or 32; re-lays out and rebuilds the lists; schedules 2 and 3 run as
  * schedule 0 at 32), and the relative Verlet margin

@@ -14,6 +14,10 @@ For every global term of an :class:`~mjolnir_b200.engine.Engine` it picks
     requests per batch (1, 2, 4) and, in the mixed form, full or half lists;
   * the lanes per particle of the list build (4, 8, 16, 32), by timing whole
     steps at the chosen margin and shape.
+An arena that steps many steps in one launch (``Engine.step_path() == 2``)
+does not run the pair launches, so its shape is chosen by timing whole steps
+over what that launch honours: the threads per particle, full or half lists and
+the list layout (schedule 0 or 5).
 In the mixed form none of the choices changes a result: the fixed-point force
 sums do not depend on list order or length, and the lists are the same.  The engine's systems keep stepping
 while the tuner measures (the tuning run is part of the warm-up).
@@ -93,7 +97,30 @@ def _apply(eng, term, shape):
     eng.set_pair_unroll(term, shape[2])
 
 
+def _in_one_launch(eng) -> bool:
+    return getattr(eng, "step_path", lambda: 1)() == 2
+
+
+def _tune_shape_by_steps(eng, term, tpps, schedules, steps: int = 60, warm: int = 20):
+    """The shape as the engine has it is kept unless another is 1 % faster."""
+    mixed = eng.precision == "mixed"
+    current = (eng.get_pair_schedule(term), eng.get_threads_per_particle(term), 1,
+               eng.get_half_lists(term) if mixed else False)
+    cands = [(s, p, 1, h) for h in ((False, True) if mixed else (False,)) for s in schedules if s in (0, 5)
+             for p in tpps if s == 0 or p >= 8]
+    best = None
+    for shape in [current] + [c for c in cands if c != current]:
+        _apply(eng, term, shape)
+        eng.step(warm)
+        ms = _time_steps(eng, steps)
+        if best is None or ms < (0.99 * best[0] if best[1] == current else best[0]):
+            best = (ms, shape)
+    return best[1]
+
+
 def _tune_shape(eng, term, tpps, unrolls, schedules):
+    if _in_one_launch(eng):
+        return _tune_shape_by_steps(eng, term, tpps, schedules)
     best = None
     # half lists (mixed form): half the list words and pair evaluations, plus
     # integer atomics for the partners' shares -- a gain where few listed

@@ -95,3 +95,47 @@ def test_margin_choice_prefers_the_narrowest_within_one_percent(monkeypatch):
     choice = autotune.tune(e, terms=("exv",), margins=tuple(step_ms))
     assert choice["exv"]["margin"] == 0.3 and e.margin == 0.3
     assert choice["exv"]["build_lanes"] == 16 and e.lanes == 16
+
+
+class OneLaunchEngine(FakeEngine):
+    """An arena that steps many steps in one launch: whole steps are timed."""
+
+    def __init__(self, precision, cost):
+        super().__init__(precision, cost)
+        self.steps = 0
+
+    def step_path(self):
+        return 2
+
+    def step(self, n):
+        self.steps += n
+
+    def get_pair_schedule(self, term):
+        return self.state["schedule"]
+
+    def get_half_lists(self, term):
+        return self.state["half"]
+
+    def time_kernel(self, term, reps=10):
+        raise AssertionError("the pair launch is not part of these steps")
+
+
+@pytest.mark.parametrize("precision", ["mixed", "fp64"])
+def test_arenas_of_one_launch_are_tuned_by_steps(precision, monkeypatch):
+    def timed(e, nsteps):
+        key = (e.state["schedule"], e.state["tpp"], e.state["unroll"], e.state["half"])
+        e.tried.append(key)
+        return e.cost(key)
+
+    monkeypatch.setattr(autotune, "_time_steps", timed)
+    fast = (5, 16, 1, precision == "mixed")
+    e = OneLaunchEngine(precision, lambda k: 0.5 if k == fast else 1.0)
+    e.state["tpp"] = 8
+    assert autotune._tune_shape(e, "dh", (1, 2, 4, 8, 16, 32), (1, 2, 4), (0, 1, 2, 3, 4, 5)) == fast
+    assert e.tried[0] == (0, 8, 1, False) and len(set(e.tried)) == len(e.tried) and e.steps > 0
+    assert all(k[0] in (0, 5) and k[2] == 1 and (k[0] == 0 or k[1] >= 8) for k in e.tried)
+    assert any(k[3] for k in e.tried) == (precision == "mixed")
+    # within 1 % of the shape it has: kept
+    e = OneLaunchEngine(precision, lambda k: 1.0 if k == (0, 8, 1, False) else 0.995)
+    e.state["tpp"] = 8
+    assert autotune._tune_shape(e, "dh", (1, 2, 4, 8, 16, 32), (1, 2, 4), (0, 5)) == (0, 8, 1, False)
