@@ -9,9 +9,10 @@ namespace mjg {
 
 // Single-instruction forms of the mixed form's reciprocal root and power of
 // two.  Squared distances and exponents of listed pairs are normal numbers, for
-// which these round as the general forms do, which spend as many instructions
-// again on subnormal ones; a subnormal squared distance gives an infinite force
-// either way, which the fixed-point range check reports.
+// which these give the floats of the general forms (rsqrtf, __expf, __frcp_rn: every
+// mantissa from 2^-60 to 2^60, tests/test_gpu_fast_math.py), which spend as many
+// instructions again on subnormal ones.  A subnormal or zero squared distance ends
+// in an infinite or NaN force, which the fixed-point range check reports.
 __device__ __forceinline__ float rsqrt_approx(float x)
 {
     float y;
@@ -24,9 +25,8 @@ __device__ __forceinline__ float exp2_approx(float x)
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
-// 1 / x: the hardware's approximation and one Newton step, r + r (1 - x r),
-// which leaves the rounding of the last product-sum (at most 1 ulp, and the
-// nearest float in nearly all cases).
+// 1 / x: the hardware's approximation and one Newton step, r + r (1 - x r), whose
+// residual is exact in the fused product-sum: the nearest float.
 __device__ __forceinline__ float reciprocal(float x)
 {
     float r;
