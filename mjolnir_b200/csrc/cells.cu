@@ -36,7 +36,7 @@ constexpr int CHUNK = 256;          // items per work chunk
 constexpr int GRID = 148 * 8;       // persistent grid: 8 blocks of 256 per SM
 constexpr int CLEAR_GRID = 148;     // the clearing launch: its last block finishes the rebuild
 
-// work counters in t.work: [0] participant chunks, [1] cell chunks, [3] blocks of the last launch done
+// work counters in t.work: [0] participant chunks, [1] cell chunks, [2] blocks of the last launch done
 
 // one block per system
 __global__ void __launch_bounds__(128) k_plan(Arena a, int g, TermArrays t, int force_all)
@@ -74,7 +74,7 @@ __global__ void __launch_bounds__(TPB) k_cells_assign(Arena a, int g, TermArrays
         const int4 w = t.part_chunks[c];
         const int p = w.y + threadIdx.x;      // participant index (same range as slots)
         if(p >= w.z) {continue;}
-        bin_participant(a, t, w.x, a.sys[w.x].g[g], p);
+        bin_participant(a, t, a.sys[w.x].g[g], p);
     }
 }
 
@@ -91,7 +91,7 @@ __global__ void __launch_bounds__(TPB) k_scan_cells(Arena a, int g, TermArrays t
         const int4 ch = t.cell_chunks[c];
         const GlobalParams& G = a.sys[ch.x].g[g];
         int before = 0;
-        for(int k = threadIdx.x; k < ch.w; k += TPB) {before += t.cell_sum[chunk_sum_index(ch.x, G, k)];}
+        for(int k = threadIdx.x; k < ch.w; k += TPB) {before += t.cell_sum[chunk_sum_index(G, k)];}
         before = __reduce_add_sync(0xffffffffu, before);
         const int first = ch.y + threadIdx.x * SCAN_ITEMS;     // this thread's cells
         int v[SCAN_ITEMS];
@@ -184,11 +184,11 @@ __global__ void __launch_bounds__(TPB) k_rebuild_done(Arena a, int g, TermArrays
     {
         const int4 ch = t.cell_chunks[c];
         for(int cell = ch.y + threadIdx.x; cell < ch.z; cell += TPB) {t.cell_count[cell] = 0;}
-        if(threadIdx.x == 0) {t.cell_sum[chunk_sum_index(ch.x, a.sys[ch.x].g[g], ch.w)] = 0;}
+        if(threadIdx.x == 0) {t.cell_sum[chunk_sum_index(a.sys[ch.x].g[g], ch.w)] = 0;}
     }
     __shared__ bool last;
     __syncthreads();
-    if(threadIdx.x == 0) {last = atomicAdd(&t.work[3], 1) == (int)gridDim.x - 1;}
+    if(threadIdx.x == 0) {last = atomicAdd(&t.work[2], 1) == (int)gridDim.x - 1;}
     __syncthreads();
     if(!last) {return;}
     for(int s = threadIdx.x; s < a.nsys; s += TPB)
@@ -201,7 +201,7 @@ __global__ void __launch_bounds__(TPB) k_rebuild_done(Arena a, int g, TermArrays
             if(!forced) {G.rebuilds += 1;}   // count only reduce_margin rebuilds
         }
     }
-    if(threadIdx.x < 4) {t.work[threadIdx.x] = 0;}
+    if(threadIdx.x < 3) {t.work[threadIdx.x] = 0;}
     if(threadIdx.x == 0) {*t.any_rebuild = 0;}
 }
 

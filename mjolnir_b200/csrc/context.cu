@@ -1315,7 +1315,7 @@ void commit(mjg_context* c)
         T.cell_sum.ensure(sizeof(int) * t.ncell);
         T.cell_start.ensure(sizeof(int) * t.ncell);
         // rebuild work lists (sized for every system flagged at once)
-        T.work.ensure(sizeof(int) * 4);
+        T.work.ensure(sizeof(int) * 3);
         CK(cudaMemsetAsync(T.work.p, 0, T.work.bytes, st));
         T.part_chunks.ensure(sizeof(int4) * std::max<long long>(1, part_chunk_cap[g]));
         T.cell_chunks.ensure(sizeof(int4) * std::max<long long>(1, cell_chunk_cap[g]));

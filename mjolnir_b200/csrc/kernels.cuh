@@ -66,7 +66,7 @@ struct TermArrays {
     int*       cell_count;      // [ncell] zero between rebuilds
     int*       cell_start;      // [ncell]
     int*       cell_sum;        // [ncell] participants per chunk of cells (chunk_sum_index), zero between rebuilds
-    int*       work;            // [4] rebuild work counters
+    int*       work;            // [3] rebuild work counters
     int4*      part_chunks;     // rebuild work: participant chunks {sys, begin, end}
     int4*      cell_chunks;     // rebuild work: cell chunks
     int*       slot_part;       // [np] scratch of the rebuild: participants in cell order, then list lengths

@@ -9,12 +9,12 @@ constexpr int CELL_CHUNK = 1024;     // cells per scan item
 
 // A system's chunk sums lie where its cells do, one word per chunk: chunk k's at
 // cell cell_off + k.
-__device__ __forceinline__ int chunk_sum_index(int, const GlobalParams& G, int k) {return G.cell_off + k;}
+__device__ __forceinline__ int chunk_sum_index(const GlobalParams& G, int k) {return G.cell_off + k;}
 
 // Bins participant p of the system: its cell and its place in the cell; counts
 // the cell and the cell's chunk (one atomic per chunk and warp; the only chunk of
 // a small grid is never summed up).
-__device__ __forceinline__ void bin_participant(const Arena& a, const TermArrays& t, int sys, const GlobalParams& G, int p)
+__device__ __forceinline__ void bin_participant(const Arena& a, const TermArrays& t, const GlobalParams& G, int p)
 {
     const double4 r = a.pos[t.part_particle[p]];
     const int c = cell_coord(r.x, G, 0) + G.dims[0] * (cell_coord(r.y, G, 1) + G.dims[1] * cell_coord(r.z, G, 2));
@@ -22,7 +22,7 @@ __device__ __forceinline__ void bin_participant(const Arena& a, const TermArrays
     t.nnb[p] = atomicAdd(&t.cell_count[G.cell_off + c], 1);    // scratch until the build writes the lengths
     if(G.ncell > CELL_CHUNK)
     {
-        const int chunk = chunk_sum_index(sys, G, c / CELL_CHUNK);
+        const int chunk = chunk_sum_index(G, c / CELL_CHUNK);
         const unsigned same = __match_any_sync(__activemask(), chunk);
         if((threadIdx.x & 31) == __ffs(same) - 1) {atomicAdd(&t.cell_sum[chunk], __popc(same));}
     }

@@ -25,7 +25,6 @@ template<> struct WinT<P_MIXED> {using type = unsigned; static constexpr int wor
 
 template<int PREC>
 struct Window {
-    static constexpr bool DEFER = false;
     using T = typename WinT<PREC>::type;
     static constexpr int SIZE = 3 * WINDOW * WinT<PREC>::words;
     T* w;         // [SIZE] in shared memory; mixed: low words, then high words

@@ -108,9 +108,9 @@ struct Barrier {
 // ------------------------------------------------- bonded forces, one by one
 // Each term adds its forces to the particles directly: in a small arena the
 // block-wide window of the bonded launch would only lengthen the chain.
+struct InLine {static constexpr bool DEFER = false;};
 template<int PREC>
-struct DirectAdd {
-    static constexpr bool DEFER = false;   // mixed form
+struct DirectAdd : InLine {
     __device__ __forceinline__ void add(void* force, int i, double fx, double fy, double fz)
     {
         Window<PREC>::global_add(force, i, fx, fy, fz);
@@ -227,7 +227,7 @@ __device__ __forceinline__ bool rebuild(const Arena& a, const TermArrays& t, ull
         k = e;
         if(!locate(mask, k, s, nslot)) {break;}
         const GlobalParams& P = a.sys[s].g[g];
-        bin_participant(a, t, s, P, P.slot_off + k);
+        bin_participant(a, t, P, P.slot_off + k);
     }
     if(!bar.sync()) {return false;}
     // first slot of each cell: one block per chunk of cells; the sums of the
@@ -239,7 +239,7 @@ __device__ __forceinline__ bool rebuild(const Arena& a, const TermArrays& t, ull
         if(!locate(mask, k, s, [&](int x) {return (a.sys[x].g[g].ncell + CELL_CHUNK - 1) / CELL_CHUNK;})) {break;}
         const GlobalParams& q = a.sys[s].g[g];
         int before = 0;
-        for(int c = threadIdx.x; c < k; c += RT) {before += t.cell_sum[chunk_sum_index(s, q, c)];}
+        for(int c = threadIdx.x; c < k; c += RT) {before += t.cell_sum[chunk_sum_index(q, c)];}
         before = __reduce_add_sync(0xffffffffu, before);
         const int cell = k * CELL_CHUNK + threadIdx.x;
         const int v = cell < q.ncell ? t.cell_count[q.cell_off + cell] : 0;
@@ -302,7 +302,7 @@ __device__ __forceinline__ void clear_cells(const Arena& a, const TermArrays& t,
         const GlobalParams& q = a.sys[s].g[g];
         for(int c = G.thread; c < q.ncell; c += G.nthread) {t.cell_count[q.cell_off + c] = 0;}
         const int nc = (q.ncell + CELL_CHUNK - 1) / CELL_CHUNK;
-        for(int c = G.thread; c < nc; c += G.nthread) {t.cell_sum[chunk_sum_index(s, q, c)] = 0;}
+        for(int c = G.thread; c < nc; c += G.nthread) {t.cell_sum[chunk_sum_index(q, c)] = 0;}
     }
 }
 
