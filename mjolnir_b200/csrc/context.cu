@@ -294,9 +294,11 @@ void enqueue_forces(mjg_context* c, const Arena& a, bool nf, bool ne)
 // launches add with integer atomics (exact in any order), so all branches may
 // overlap; the FP64 form adds its pair forces after the join, one term after
 // the other.
-// arenas with at most this many systems carrying a term put that term's
-// rebuild behind a graph conditional (measured: a 10,000-bead melt alone steps
-// 10-18 % faster, a 256-system batch 5 % slower with it)
+// Captured arenas with at most this many systems carrying a term put that term's
+// rebuild behind a graph conditional.  Measured, us per step without / with it: one
+// melt of 115,000 beads 57 / 49, four melts of 30,000 57 / 51, eight of 15,000 57 / 53,
+// the 262,144- and 1,048,576-bead fluids 302 / 297 and 1,092 / 1,086; a 256-system
+// batch, where some system rebuilds at nearly every step, was 5 % slower with it.
 constexpr int GATE_MAX_SYSTEMS = 4;
 
 void enqueue_step_body(mjg_context* c, bool kick, bool capturing)
