@@ -575,7 +575,9 @@ def run_b200(args, ws, rank, local, pg):
                 "timing": "CUDA events per launch on the library stream, L2 evicted before each launch",
                 "ms_per_launch": k["ms"], "pairs_in_cutoff": k["pcut"],
                 "algorithmic_bytes": k["bytes"], "other": {t: kern[t] for t in kern if t != dom},
-                "local_ms_per_launch": local_ms}
+                "local_ms_per_launch": local_ms,
+                "local_note": "each bonded term alone; the mixed step joins the three in one launch "
+                              "(profiles/k_local_records_batch256_mixed.md)"}
 
     # ---- plain single-system FP64 path: every system of the batch, one at a time
     plain = None
