@@ -67,8 +67,10 @@ MJG_API const char* mjg_last_error(const mjg_context* ctx);
  * the SMs it runs on until it ends (about 10 ms at most); 2: it replays captured
  * graphs in small arenas too; 0: it launches every kernel of every step. */
 MJG_API int  mjg_context_set_graphs(mjg_context* ctx, int enable);
-/* How mjg_step runs the committed arena: 0 separate launches, 1 captured
- * graphs, 2 many steps in one launch. */
+/* How mjg_step runs the committed arena in a long simulation: 0 separate
+ * launches, 1 captured graphs (of arenas not much larger than those of 2, the
+ * first few hundred steps after a commit still run in one launch, which saves
+ * capturing graphs for them), 2 many steps in one launch. */
 MJG_API int  mjg_context_step_path(mjg_context* ctx, int* path);
 /* Options: the per-step work of mjg_step is also checked for list overflow
  * and rolled back when it happens (default 1). */

@@ -191,6 +191,7 @@ struct mjg_context {
     int sms = 0;                            // SMs of the device
     int64_t wait_cycles = mjg::RUN_WAIT_CYCLES;   // limit of a wait inside the multi-step kernel
     int run_blocks = 0;                     // blocks of the multi-step kernel, 0: by the arena's size
+    int64_t uncaptured = 0;                 // steps of the multi-step kernel since the graphs became void
     bool run_refused = false;               // the runtime refused its launch: this arena steps by graphs
     bool torn = false;                      // a chunk stopped half-way and could not be rolled back
     double* h_pinned = nullptr;             // page-locked host staging (state, forces)
@@ -275,6 +276,7 @@ void release_graph(mjg_context* c)
     if(c->graph4_exec) {cudaGraphExecDestroy(c->graph4_exec); c->graph4_exec = nullptr;}
     if(c->graph4) {cudaGraphDestroy(c->graph4); c->graph4 = nullptr;}
     c->graph_dirty = true;
+    c->uncaptured = 0;
 }
 
 // ------------------------------------------------------------ schedule
@@ -944,6 +946,19 @@ bool run_fits(long long n, int nsys, int precision)
     return n > 0 && n <= run_max_particles(precision) && nsys <= RUN_MAX_SYSTEMS;
 }
 
+// Between the mixed form's line and this size the graphs gain up to 10 us per step,
+// and capturing them after a commit or a change of shape costs 1.3 ms (40 melts of
+// 115,000 beads, first 100 steps: 5.7 ms in the multi-step kernel, 7.0 with the
+// capture; later ones 6.2 and 6.1): the first RUN_UNCAPTURED steps since then run in
+// the multi-step kernel.
+constexpr long long RUN_UNCAPTURED_MAX_PARTICLES = 131072;
+constexpr int64_t RUN_UNCAPTURED = 256;
+bool steps_before_capture(long long n, int nsys, int precision)
+{
+    return precision == P_MIXED && n > run_max_particles(precision) && n <= RUN_UNCAPTURED_MAX_PARTICLES &&
+           nsys <= RUN_MAX_SYSTEMS;
+}
+
 // Steps per launch.  A launch holds every SM it runs on until it ends, so this
 // bounds how long other work on the GPU waits: about 10 ms (200 beads 1,024 steps
 // of 8 us, 10,000-bead melt 838 of 12, 90,000 beads 93 of 42 to 125).  A launch
@@ -1563,9 +1578,17 @@ void clear_stalled(mjg_context* c)
     }
 }
 
+// the path of a long simulation (mjg_context_step_path)
 bool steps_in_one_launch(const mjg_context* c)
 {
     return c->graphs == 1 && run_fits(c->arena.n, c->arena.nsys, c->precision) && !c->run_refused;
+}
+// the path of a call of nsteps
+bool call_in_one_launch(const mjg_context* c, int64_t nsteps)
+{
+    return steps_in_one_launch(c) ||
+           (c->graphs == 1 && !c->run_refused && c->graph_dirty && c->uncaptured + nsteps <= RUN_UNCAPTURED &&
+            steps_before_capture(c->arena.n, c->arena.nsys, c->precision));
 }
 
 void run_steps(mjg_context* c, int64_t nsteps)
@@ -1576,7 +1599,7 @@ void run_steps(mjg_context* c, int64_t nsteps)
     bool stalled = false;                           // the chunk's waits ran out once: step by launches instead
     for(int attempt = 0; attempt < 8; ++attempt)
     {
-        const bool multi = steps_in_one_launch(c) && !stalled;
+        const bool multi = call_in_one_launch(c, nsteps) && !stalled;
         if(c->rollback && !multi)                   // the multi-step kernel copies the state itself
         {
             CK(cudaMemcpyAsync(c->b_sys.p, c->d_sys.p, c->d_sys.bytes, cudaMemcpyDeviceToDevice, st));
@@ -1659,7 +1682,11 @@ void run_steps(mjg_context* c, int64_t nsteps)
         else
         {
             check_status(c, overflow);
-            if(!overflow) {return;}
+            if(!overflow)
+            {
+                if(multi) {c->uncaptured += nsteps;}
+                return;
+            }
             if(!c->rollback) {throw Error(MJG_ESTATE, "a Verlet list overflowed (enable rollback)");}
         }
         // roll back, grow the lists, rebuild, retry

@@ -161,7 +161,7 @@ void launch_set_force(const Arena& a, const double* src, long long first, long l
                       cudaStream_t s);
 
 // Many steps of a small arena in one launch (run.cu).
-constexpr int RUN_MAX_SYSTEMS = 64;
+constexpr int RUN_MAX_SYSTEMS = 64;  // the bits of its word of systems to rebuild
 constexpr int RUN_CLUSTER_MAX = 8;   // blocks up to which the launch is one cluster (the portable size)
 constexpr int RUN_LEFT = 32;         // in a line of its own
 constexpr long long RUN_WAIT_CYCLES = 2LL << 30;   // default wait_cycles: about a second

@@ -5,21 +5,23 @@
 // cooperatively) walks the step's phases itself -- integrator pass, margin
 // bookkeeping, list rebuilds of the systems that need them, forces -- with a
 // barrier between phases, so a step without a rebuild costs two barriers
-// instead of a chain of dependent graph nodes.  What bounds it is the latency
+// instead of a chain of dependent graph nodes.  (The arenas it takes: run_fits in
+// context.cu.)  What bounds it is the latency
 // of each phase's chain of dependent loads plus the barriers (about a
 // microsecond each over the whole GPU, less within one cluster), so the work
 // of a phase is spread warp by warp over every SM: consecutive warp items go
 // to different blocks.  The arithmetic is that of the step's launches
 // (advance_particle, PairEval, the bonded formulas, the list builds), so in
 // the mixed form, whose force sums are exact, a chunk gives the same bits
-// either way.
+// either way.  The FP64 form adds a particle's terms in the launches' order
+// (run_force).
 //
-// Measured (graph of launches / this kernel, us per step): 200-bead chain 23 /
-// 9.4, 4,096-particle Lennard-Jones fluid 33 / 17.6 mixed and 32 / 16.9 FP64,
-// 2,997-bead melt 24.6 / 12.1, 10,000-bead melt FP64 31 / 14.8.  Of the
-// Lennard-Jones fluid's 17.6 the integrator pass takes 1.8, its barrier 1.3,
-// the margins 0.8, the forces 5.7, the second barrier with the noise drawn
-// meanwhile 1.8, and a twelfth of a rebuild 3.1.
+// Measured (graph of launches / this kernel, us per step, calls of 50 to 100
+// steps): 200-bead chain 23 / 8.6, 4,096-particle Lennard-Jones fluid 33 / 16.7
+// mixed and 32 / 16.0 FP64, 2,997-bead G-JF melt 26 / 10.9, 10,000-bead melt FP64
+// 30 / 14.6.  Of the Lennard-Jones fluid's 16.7 the integrator pass takes 1.8, its
+// barrier 1.6, the margins 0.7, the forces 5.4, the second barrier with the noise
+// drawn meanwhile 2.3, and a twelfth of a rebuild 3.5.
 //
 // Every load here is a plain one: lists, slot coordinates and cells are
 // rewritten during the launch, which the read-only path must not see.

@@ -79,19 +79,29 @@ def test_launch_shapes_fp64(graphs):
 
 
 def test_the_line_between_the_paths():
-    """At the largest arena that steps in one launch, and one particle above it."""
-    for precision, n, path in (("mixed", 90000, 2), ("mixed", 90001, 1), ("fp64", 90001, 2)):
+    """At the largest arena that steps in one launch, and one particle above it: the mixed form's first steps
+    there still run in one launch, and again after a commit; then the graphs are captured."""
+    for precision, n, path in (("mixed", 90000, 2), ("mixed", 90001, 1), ("mixed", 131073, 1), ("fp64", 90001, 2)):
         d = S.bead_fluid(n=n, density=0.003, seed=8, dt=0.6, margin=0.05)
         outs = []
         for graphs in (True, False):
             e = Engine(precision, graphs=graphs)
             sid = e.add_system(d)
             e.commit()
+            single = []
+            for k in (15, 100, 142, 5, 0, 20):
+                if k == 0:
+                    e.commit()
+                    continue
+                n0 = e.launch_count()
+                e.step(k)
+                single.append(e.launch_count() - n0 <= 2)       # at most two launches of the multi-step kernel
             if graphs:
                 assert e.step_path() == path
-            e.step(15)
+                early = path == 2 or n <= 131072
+                assert single == [early, early, path == 2, path == 2, early]
             assert e.rebuild_count(sid, "exv") > 0
             outs.append(e.state(sid))
             e.close()
         for x, y in zip(*outs):
-            assert np.array_equal(x, y) if precision == "mixed" else np.abs(x - y).max() <= 1e-9 * np.abs(y).max()
+            assert np.array_equal(x, y) if precision == "mixed" else np.abs(x - y).max() <= 1e-7 * np.abs(y).max()
