@@ -458,6 +458,7 @@ void alloc_lists(mjg_context* c, int g, int cap)
     T.nbr.ensure(sizeof(int) * list_words(cap) * (size_t)(T.t.np > 0 ? T.t.np : 1));
     T.t.nbr = T.nbr.as<int>();
     T.t.cap = cap;
+    T.t.words = (int)list_words(cap);
     T.cap_alloc = cap;
     release_graph(c);
 }
@@ -1410,6 +1411,7 @@ void commit(mjg_context* c)
             T.nbr.bytes = sizeof(int) * list_words(keep) * (size_t)np;
             t.nbr = T.nbr.as<int>();
             t.cap = keep;
+            t.words = (int)list_words(keep);
             if(!T.tpp_fixed) {t.tpp = prev_tpp;}
         }
         else
@@ -2373,7 +2375,7 @@ int mjg_neighbors(mjg_context* c, int sys, int term, int64_t* pairs, int64_t cap
     std::vector<int> nnb(t.np), part(t.np);
     CK(cudaMemcpy(nnb.data(), t.nnb, sizeof(int) * t.np, cudaMemcpyDeviceToHost));
     CK(cudaMemcpy(part.data(), t.slot_particle, sizeof(int) * t.np, cudaMemcpyDeviceToHost));
-    std::vector<int> all(list_words(t.cap) * (size_t)t.np);
+    std::vector<int> all((size_t)t.words * (size_t)t.np);
     if(!all.empty())
     {
         CK(cudaMemcpy(all.data(), t.nbr, sizeof(int) * all.size(), cudaMemcpyDeviceToHost));
@@ -2383,7 +2385,7 @@ int mjg_neighbors(mjg_context* c, int sys, int term, int64_t* pairs, int64_t cap
     {
         for(int k = 0; k < nnb[q]; ++k)
         {
-            const int r = all[(size_t)nbr_pos(k, q, t.np, t.tpp, t.cap, t.slot_major)];
+            const int r = all[(size_t)nbr_pos(k, q, t.np, t.tpp, t.words, t.slot_major)];
             const int64_t i = part[q] - s.off, j = part[r] - s.off;
             if(t.half) {out.emplace_back(std::min(i, j), std::max(i, j));}   // each pair listed once
             else if(i < j) {out.emplace_back(i, j);}

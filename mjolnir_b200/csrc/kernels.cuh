@@ -39,7 +39,9 @@ struct TermArrays {
     int        on;
     long long  np;              // participants (= slots)
     int        ncell;           // total cells over all systems
-    int        cap;             // neighbour capacity per slot (a multiple of tpp)
+    int        cap;             // longest list that a build writes whole
+    int        words;           // words of the neighbour buffer per slot (a multiple of 32, not below cap): the
+                                // slots' distance in the slot-major layout, also where cap is lowered
     int        tpp;             // threads per slot of the pair kernel (1, 2, 4, 8, 16, 32)
     int        unroll;          // partners requested per batch by the force launch (1, 2, 4)
     int        schedule;        // force launch: 0 = slot per tpp threads, 1 = warp-balanced (mixed),

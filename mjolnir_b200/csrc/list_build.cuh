@@ -290,7 +290,7 @@ __device__ __forceinline__ void build_list_group(const Arena& a, int g, const Te
         {
             const int k = count + __popc(m & ((1u << lane) - 1u));
             // nbr_pos with the power of two as a shift
-            if(k < cap) {t.nbr[t.slot_major ? (long long)s * cap + k : ((((long long)(k >> lt) * np + s) << lt) + (k & (t.tpp - 1)))] = q;}
+            if(k < cap) {t.nbr[t.slot_major ? (long long)s * t.words + k : ((((long long)(k >> lt) * np + s) << lt) + (k & (t.tpp - 1)))] = q;}
         }
         count += __popc(m);
         q = qn;

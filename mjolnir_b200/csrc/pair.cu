@@ -44,7 +44,7 @@ __global__ void k_count_cut(Arena a, TermArrays t, int sys_filter, unsigned long
         const int n = t.nnb[s];
         for(int k = 0; k < n; ++k)
         {
-            const int q = t.nbr[nbr_pos(k, s, t.np, t.tpp, t.cap, t.slot_major)];
+            const int q = t.nbr[nbr_pos(k, s, t.np, t.tpp, t.words, t.slot_major)];
             if(q <= s) {continue;}
             const double4 pj = t.slot_pd[q];
             double dx = pj.x - pi.x, dy = pj.y - pi.y, dz = pj.z - pi.z;

@@ -111,15 +111,15 @@ __global__ void __launch_bounds__(TPB, 4) k_pair(Arena a, TermArrays t)
     if(active && (!SORT || head.n > 0))    // a sorted group knows that its list is empty
     {
         // word k = lg + r TPP of the slot's list: blocked layout, rows np TPP
-        // words apart; slot-major layout, the slot's cap words in a row, the
-        // whole list requested into L2 (16-byte aligned: cap is a multiple of
-        // 32 words) before the walk starts
+        // words apart; slot-major layout, the slot's words in a row, the
+        // whole list requested into L2 (16-byte aligned: a multiple of 32
+        // words per slot) before the walk starts
         const bool sm = t.slot_major != 0;
         const long long rs = sm ? TPP : t.np * TPP;
-        const int* __restrict__ nbr = t.nbr + (sm ? s * t.cap : s * TPP) + lg;
+        const int* __restrict__ nbr = t.nbr + (sm ? s * t.words : s * TPP) + lg;
         const double4* __restrict__ pd = t.slot_pd;
         // the slot's coordinates, particle and first list word are requested
-        // with its head (every slot owns cap >= TPP words; a word past the
+        // with its head (every slot owns at least TPP words; a word past the
         // length is never used as an index), so the walk starts one load
         // latency after the launch
         const double4 self = load_pd(pd + s);
@@ -127,7 +127,7 @@ __global__ void __launch_bounds__(TPB, 4) k_pair(Arena a, TermArrays t)
         particle = t.slot_particle[s];
         if(!SORT) {head = slot_head(a, t, s);}
         const int n = head.n;
-        if(sm && lg == 0 && n > 0) {bulk_prefetch_l2(t.nbr + s * t.cap, (unsigned)((n + 3) / 4) * 16u);}
+        if(sm && lg == 0 && n > 0) {bulk_prefetch_l2(t.nbr + s * t.words, (unsigned)((n + 3) / 4) * 16u);}
         if(n > 0)
         {
         const PairEval<PREC, G, NF, NE, PER, HALF> eval(a, t, s, head.sys, self);
@@ -253,7 +253,7 @@ __global__ void __launch_bounds__(TPB, 4) k_pair_vec(Arena a, TermArrays t)
     }
     if(s >= t.np || (SORT && head.n == 0)) {return;}   // an empty list (frequent in half lists): nothing to add
     // the slot's coordinates, particle and first block of words are requested
-    // with its head (every slot owns cap >= L words; words past the length are
+    // with its head (every slot owns at least L words; words past the length are
     // never used as indices)
     const double4 self = load_pd(t.slot_pd + s);
     int q[L];

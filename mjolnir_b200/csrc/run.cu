@@ -331,7 +331,7 @@ __device__ __forceinline__ void pair_item(const Arena& a, const TermArrays& t, d
         const long long np = t.np;
         const bool sm = t.slot_major != 0;
         const long long rs = sm ? tpp : np * tpp;
-        const int* nbr = t.nbr + (sm ? s * t.cap : s * tpp) + lg;
+        const int* nbr = t.nbr + (sm ? s * t.words : s * tpp) + lg;
         const double4* pd = t.slot_pd;
         const double4 self = load_pd(pd + s);
         const int first = nbr[0];

@@ -153,3 +153,24 @@ def test_overflow_in_a_later_launch_rolls_the_chunk_back():
     got, redone = states(5000, cap)
     assert plain == 5 and redone > 5
     assert all(np.array_equal(x, y) for x, y in zip(got, want))
+
+
+@pytest.mark.parametrize("graphs", [True, 2, False])
+def test_capacity_of_contiguous_lists(graphs):
+    """Lists stored particle by particle keep their distance when the capacity is lowered below their length, and
+    take a capacity that is no multiple of a copy's 16 bytes: the lists stay readable, and the overflow is met."""
+    d = S.lj_fluid(n=1000, density=0.8, margin=0.1, seed=44)
+    want = None
+    for schedule, caps in ((0, ()), (5, (8,)), (5, (333, 9))):
+        e = Engine("mixed", graphs=graphs)
+        sid = e.add_system(d)
+        e.commit()
+        e.set_pair_schedule("lj", schedule)
+        pairs = e.neighbors(sid, "lj")
+        for cap in caps:
+            e.debug_set_list_capacity("lj", cap)
+            assert np.array_equal(e.neighbors(sid, "lj"), pairs)
+        got = [x for k in (1, 300) for x in (e.step(k), *e.state(sid))[1:]]
+        e.close()
+        want = want or got
+        assert all(np.array_equal(x, y) for x, y in zip(got, want))
